@@ -31,6 +31,7 @@ typedef unsigned long long uint64_t;
 #include "rf_params.h"
 
 #define RF_DEV static __device__ __forceinline__
+#define RF_DEV_MEMBER __device__ __forceinline__
 
 // ---------------------------------------------------------------------------------------
 // column loads.  rf_ld reads a column at the scanned row: each value is read once by a query,
@@ -385,6 +386,44 @@ RF_DEV unsigned long long rf_df_slot_to_f64(unsigned long long w)
 {
     const double hi = (double)__uint_as_float((unsigned)w), lo = (double)__uint_as_float((unsigned)(w >> 32));
     return rf_f2u(__dadd_rn(hi, lo));
+}
+
+// ---------------------------------------------------------------------------------------
+// First i of [lo, hi) for which before(i) is false (before: true, then false), hi where there is
+// none; the whole warp searches, 32 probes a step, so a search of n elements waits on
+// log32(n) loads instead of log2(n).  Never probes outside [lo, hi).
+// ---------------------------------------------------------------------------------------
+template <class F>
+RF_DEV long long rf_warp_search(long long lo, long long hi, F before)
+{
+    const int lane = threadIdx.x & 31;
+    while (lo < hi) {
+        const long long step = (hi - lo + 31) >> 5;
+        const long long i = lo + (lane + 1) * step - 1;
+        const unsigned m = __ballot_sync(0xffffffffu, i < hi && before(i));
+        const int c = m == 0xffffffffu ? 32 : __ffs(~m) - 1;  // probes before the answer
+        const long long e = lo + (c + 1) * step - 1;
+        lo += c * step;
+        if (lo > hi) lo = hi;
+        hi = e < hi ? e : hi;
+    }
+    return lo;
+}
+
+// the words of an 8-byte aligned struct from the lane `off` below
+template <class A>
+RF_DEV A rf_shfl_up(const A& a, int off)
+{
+    static_assert(sizeof(A) % 8 == 0, "whole words");
+    union U {
+        A a;
+        unsigned long long w[sizeof(A) / 8];
+        RF_DEV_MEMBER U() {}
+    } x, y;
+    x.a = a;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(A) / 8); i++) y.w[i] = __shfl_up_sync(0xffffffffu, x.w[i], off);
+    return y.a;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -536,3 +536,191 @@ RF_DEV void rf_mat_write_all(const RfParams& P, int ncols)
         rf_mat_write_all<T>(P, NCOLS);                                                                   \
     }
 #endif  // RF_MATERIALIZE
+
+// ---------------------------------------------------------------------------------------
+// Template 4: segmented reduce over run-end encoded rows (an Op over a 2-d vector whose output
+// reduces each run, loopgen.cpp:34-38, 206-269).
+//   The fragment defines RfAcc and its functions as template 1 does, RF_SEG_M (items of a tile, a
+//   multiple of RF_SEG_T), rf_seg_runs(P) (the run-end column), struct RfSegRows (RF_SEG_M rows of
+//   the columns a row reads), rf_seg_stage(P, r, i, S) and rf_seg_row(P, r, i, S, A).
+//   P.aux_n0: rows, P.aux_n1: tiles; (long long*)P.aux4: the run each tile starts in (tiles + 1);
+//   (RfAcc*)P.aux5: a state per run, then a state per tile (its rows after its last run end).
+// Rows and run ends are merged into one sequence - run end j comes after the rows before it, at
+// position ends[j] + j - and cut into tiles of RF_SEG_M items and threads of RF_SEG_M / RF_SEG_T,
+// so every thread does the same work however long the runs are (Merrill and Garland, merge-based
+// sparse matrix-vector product, SC16).  A run inside a thread is stored by it; a run that spans
+// threads is joined by a segmented scan over the block, one that spans tiles by rf_seg_fix; all in
+// row order, by the tiles alone, so the bits do not depend on the scheduling.  Bound by reading
+// the rows: they are staged through shared memory, whole sectors a warp, and so are the run ends.
+// (20M rows of one double in 2M Zipf(1.1) runs: 2.37 ms a call with a thread to each 256 rows of a
+// run and one thread folding a run's pieces in turn, of which 1.94 ms were those folds; 0.33 ms so.)
+// ---------------------------------------------------------------------------------------
+#ifdef RF_SEG_REDUCE
+RF_DEV long long rf_seg_end(const RfParams& P, long long run)
+{
+    const long long e = (long long)__ldg(rf_seg_runs(P).run_ends + run);
+    return e < P.aux_n0 ? e : P.aux_n0;
+}
+
+// the tile's first run: the run ends before item d
+extern "C" __global__ void __launch_bounds__(256) rf_seg_part(const __grid_constant__ RfParams P)
+{
+    const long long t = (blockIdx.x * 256ll + threadIdx.x) >> 5;
+    if (t > P.aux_n1) return;
+    const long long n = rf_seg_runs(P).len, d = t * RF_SEG_M;
+    const long long x = rf_warp_search(0, n, [&](long long j) { return rf_seg_end(P, j) + j < d; });
+    if ((threadIdx.x & 31) == 0) ((long long*)P.aux4)[t] = x;
+}
+
+// segmented scan over the block: `closed`/`a` of this thread -> the state that the rows of the
+// threads before it carry into it (those since the last run end); the block's own carry out in
+// *out.  A state combines with what precedes it on the left.
+template <int T>
+RF_DEV RfAcc rf_seg_carry(const RfParams& P, bool closed, const RfAcc& a, RfAcc* warp_a, unsigned char* warp_f, RfAcc* out)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    RfAcc v = a;
+    bool f = closed;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        RfAcc u = rf_shfl_up(v, off);
+        const bool uf = __shfl_up_sync(0xffffffffu, (int)f, off) != 0;
+        if (lane >= off) {
+            if (!f) {
+                rf_acc_combine(u, v);
+                v = u;
+            }
+            f = f || uf;
+        }
+    }
+    if (lane == 31) {
+        warp_a[warp] = v;
+        warp_f[warp] = f;
+    }
+    __syncthreads();
+    // what the warps before this one carry in, then this warp's lanes before this one
+    RfAcc c;
+    rf_acc_init(P, c);
+    for (int w = 0; w < warp; w++) {
+        if (warp_f[w]) c = warp_a[w];
+        else rf_acc_combine(c, warp_a[w]);
+    }
+    if (threadIdx.x == T - 1 && out) {
+        RfAcc o = c;
+        if (f) o = v;
+        else rf_acc_combine(o, v);
+        *out = o;
+    }
+    RfAcc u = rf_shfl_up(v, 1);
+    const bool uf = __shfl_up_sync(0xffffffffu, (int)f, 1) != 0;
+    if (lane > 0) {
+        if (uf) c = u;
+        else rf_acc_combine(c, u);
+    }
+    return c;
+}
+
+extern "C" __global__ void __launch_bounds__(RF_SEG_T) rf_seg_reduce(const __grid_constant__ RfParams P)
+{
+    constexpr int T = RF_SEG_T, K = RF_SEG_M / RF_SEG_T;
+    __shared__ RfSegRows S;
+    __shared__ int ends[RF_SEG_M + 1];  // run ends of the tile, relative to its first row
+    __shared__ RfAcc warp_a[T / 32];
+    __shared__ unsigned char warp_f[T / 32];
+    const long long* part = (const long long*)P.aux4;
+    RfAcc* res = (RfAcc*)P.aux5;
+    const long long n = rf_seg_runs(P).len;
+    const long long total = (n > 0 ? rf_seg_end(P, n - 1) : 0) + n;  // items
+    const long long tile = blockIdx.x;
+    long long d0 = tile * RF_SEG_M, d1 = d0 + RF_SEG_M;
+    if (d0 > total) d0 = total;
+    if (d1 > total) d1 = total;
+    const long long xa = __ldg(part + tile), xb = __ldg(part + tile + 1);
+    // (bounded for columns whose run ends are out of order, too: never more than a tile's)
+    int nx = (int)(xb - xa < 0 ? 0 : xb - xa > RF_SEG_M ? RF_SEG_M : xb - xa);
+    const long long ra = d0 - xa;
+    int nr = (int)(d1 - d0) - nx;
+    if (nr < 0 || ra < 0 || ra + nr > P.aux_n0) nr = 0;
+    for (int i = threadIdx.x; i < nr; i += T) rf_seg_stage(P, ra + i, i, S);
+    for (int i = threadIdx.x; i < nx; i += T) ends[i] = (int)(rf_seg_end(P, xa + i) - ra);
+    __syncthreads();
+    // the thread's first item: the run ends before it
+    const int items = nr + nx;
+    int at = (int)threadIdx.x * K;
+    if (at > items) at = items;
+    int lo = at - nr > 0 ? at - nr : 0, hi = at < nx ? at : nx;
+    while (lo < hi) {
+        const int m = (lo + hi) >> 1;
+        if (ends[m] + m < at) lo = m + 1;
+        else hi = m;
+    }
+    int x = lo, r = at - lo;
+    const int first = x;
+    RfAcc A, head;
+    rf_acc_init(P, A);
+    head = A;
+    bool closed = false;
+    int e = x < nx ? ends[x] : 0x7fffffff;
+    for (int k = 0; k < K && r + x < items; k++) {
+        if (r < e && r < nr) {
+            rf_seg_row(P, ra + r, r, S, A);
+            r++;
+        } else if (x < nx) {
+            if (!closed) head = A;
+            else rf_st_words(res + xa + x, &A, (int)sizeof(RfAcc));
+            closed = true;
+            rf_acc_init(P, A);
+            x++;
+            e = x < nx ? ends[x] : 0x7fffffff;
+        }
+    }
+    RfAcc out;
+    RfAcc c = rf_seg_carry<T>(P, closed, A, warp_a, warp_f, &out);
+    if (closed) {
+        rf_acc_combine(c, head);
+        rf_st_words(res + xa + first, &c, (int)sizeof(RfAcc));
+    }
+    if (threadIdx.x == T - 1) rf_st_words(res + n + tile, &out, (int)sizeof(RfAcc));
+}
+
+// joins the runs that span tiles: the carries of the tiles since a run began, onto its state
+extern "C" __global__ void __launch_bounds__(512) rf_seg_fix(const __grid_constant__ RfParams P)
+{
+    constexpr int T = 512;
+    __shared__ RfAcc warp_a[T / 32];
+    __shared__ unsigned char warp_f[T / 32];
+    const long long* part = (const long long*)P.aux4;
+    RfAcc* res = (RfAcc*)P.aux5;
+    const long long n = rf_seg_runs(P).len, nt = P.aux_n1;
+    // a thread takes K consecutive tiles: first their carry out, then, with what is carried into
+    // them, their first runs
+    const long long K = (nt + T - 1) / T;
+    const long long t0 = threadIdx.x * K < nt ? threadIdx.x * K : nt, t1 = t0 + K < nt ? t0 + K : nt;
+    RfAcc A, b;
+    rf_acc_init(P, A);
+    bool closed = false;
+    for (long long t = t0; t < t1; t++) {
+        rf_ld_words(&b, res + n + t, (int)sizeof(RfAcc));
+        if (part[t + 1] > part[t]) {
+            closed = true;
+            A = b;
+        } else {
+            rf_acc_combine(A, b);
+        }
+    }
+    RfAcc c = rf_seg_carry<T>(P, closed, A, warp_a, warp_f, nullptr);
+    for (long long t = t0; t < t1; t++) {
+        const long long x = part[t];
+        rf_ld_words(&b, res + n + t, (int)sizeof(RfAcc));
+        if (part[t + 1] > x) {
+            RfAcc h;
+            rf_ld_words(&h, res + x, (int)sizeof(RfAcc));
+            rf_acc_combine(c, h);
+            rf_st_words(res + x, &c, (int)sizeof(RfAcc));
+            c = b;
+        } else {
+            rf_acc_combine(c, b);
+        }
+    }
+}
+#endif  // RF_SEG_REDUCE

@@ -1626,7 +1626,9 @@ private:
             }
         }
         const bool vec4 = !hl.empty() && plan_.kind == PlanKind::SCAN_REDUCE;
-        if (vec4) {
+        const bool split = vec4 || (!hl.empty() && plan_.kind == PlanKind::SEG_REDUCE);
+        row_loads_ = hl;
+        if (split) {
             row << "RF_DEV void rf_row_v(const RfParams& P, long long r, RfAcc& A";
             for (auto& h : hl) row << ", const " << h[0] << " " << h[1];
             row << ")\n{\n" << body.str();
@@ -1639,11 +1641,13 @@ private:
         row << updates;
         if (act.empty()) row << "    (void)A;\n";
         row << "}\n\n";
-        if (vec4) {
+        if (split) {
             row << "RF_DEV void rf_row(const RfParams& P, long long r, RfAcc& A)\n{\n" << hoisted;
             row << "    rf_row_v(P, r, A";
             for (auto& h : hl) row << ", " << h[1];
             row << ");\n}\n\n";
+        }
+        if (vec4) {
             row << "#define RF_VEC4 1\n";
             row << "RF_DEV void rf_row4(const RfParams& P, long long r, RfAcc& A)\n{\n";
             for (auto& h : hl) {
@@ -2314,37 +2318,45 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         }
     }
 
-    // Segmented reduce over run-end encoded rows: every run is cut into chunks of RF_SEG_CH rows
-    // (long Zipf runs spread over many threads); chunk c of run r is reduced by one thread in row
-    // order into partial[woff[r] + c]; the element functions fold a run's partials in order.
-    // woff: (long long*)P.aux4 (nruns + 1 entries), partials: (RfAcc*)P.aux5.
+    // Segmented reduce over run-end encoded rows (template 4): the row's columns as a staged struct,
+    // and the run's state as the element functions read it.  The tile is as many items as 36 KiB of
+    // shared memory hold beside their run ends, 11 a thread at most, so that six blocks fit an SM.
     void emit_seg_kernels(std::ostringstream& o, const Drive& d)
     {
-        std::string c0 = "P.t[" + std::to_string(d.slot) + "].col[0]";
-        o << "#define RF_SEG_CH 256\n";
-        o << "extern \"C\" __global__ void __launch_bounds__(256) rf_seg_count(const __grid_constant__ RfParams P)\n{\n";
-        o << "    long long* woff = (long long*)P.aux4;\n    const long long n = " << c0 << ".len;\n";
-        o << "    for (long long run = blockIdx.x * (long long)blockDim.x + threadIdx.x; run < n; run += (long long)gridDim.x * blockDim.x) {\n";
-        o << "        long long len = rf_runend(" << c0 << ", run) - rf_runend(" << c0 << ", run - 1);\n";
-        o << "        long long c = (len + RF_SEG_CH - 1) / RF_SEG_CH;\n        woff[run] = c < 1 ? 1 : c;\n    }\n}\n\n";
-        o << "extern \"C\" __global__ void __launch_bounds__(256) rf_seg_reduce(const __grid_constant__ RfParams P)\n{\n";
-        o << "    const long long* woff = (const long long*)P.aux4;\n    RfAcc* part = (RfAcc*)P.aux5;\n";
-        o << "    const long long n = " << c0 << ".len, W = woff[n];\n";
-        o << "    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < W; w += (long long)gridDim.x * blockDim.x) {\n";
-        o << "        long long lo = 0, hi = n;  // last run with woff[run] <= w\n";
-        o << "        while (hi - lo > 1) { long long mid = (lo + hi) >> 1; if (woff[mid] <= w) lo = mid; else hi = mid; }\n";
-        o << "        const long long run = lo, k = w - woff[run];\n";
-        o << "        const long long s = rf_runend(" << c0 << ", run - 1) + k * RF_SEG_CH;\n";
-        o << "        long long e = rf_runend(" << c0 << ", run);\n        if (e > s + RF_SEG_CH) e = s + RF_SEG_CH;\n";
-        o << "        RfAcc A;\n        rf_acc_init(P, A);\n        for (long long r = s; r < e; r++) rf_row(P, r, A);\n";
-        o << "        rf_st_words(part + w, &A, (int)sizeof(RfAcc));\n    }\n}\n\n";
-        o << "RF_DEV void rf_fold(const RfParams& P, long long run, RfAcc& A)\n{\n";
-        o << "    const long long* woff = (const long long*)P.aux4;\n    const RfAcc* part = (const RfAcc*)P.aux5;\n";
-        o << "    rf_acc_init(P, A);\n    for (long long w = woff[run]; w < woff[run + 1]; w++) {\n";
-        o << "        RfAcc p;\n        rf_ld_words(&p, part + w, (int)sizeof(RfAcc));\n        rf_acc_combine(A, p);\n    }\n}\n\n";
-        plan_.kernels.push_back({"rf_seg_count", 256, 0, KernelSpec::SEGCOUNT});
-        plan_.kernels.push_back({"", 0, 0, KernelSpec::SEGSCAN});
-        plan_.kernels.push_back({"rf_seg_reduce", 256, 0, KernelSpec::SEGREDUCE});
+        const int T = 256;
+        int row_bytes = 4;  // a run end
+        for (auto& h : row_loads_) row_bytes += h[0] == "bool" ? 1 : (int)size_of_ctype(h[0]);
+        const int K = std::max(1, std::min(11, 36 * 1024 / (T * row_bytes)));
+        plan_.seg_items = T * K;
+        o << "#define RF_SEG_REDUCE 1\n#define RF_SEG_T " << T << "\n#define RF_SEG_M " << T * K << "\n";
+        o << "RF_DEV const RfCol& rf_seg_runs(const RfParams& P) { return P.t[" << d.slot << "].col[0]; }\n";
+        o << "struct RfSegRows {\n";
+        for (auto& h : row_loads_) o << "    " << h[0] << " " << h[1] << "[RF_SEG_M];\n";
+        if (row_loads_.empty()) o << "    int unused;\n";
+        o << "};\nRF_DEV void rf_seg_stage(const RfParams& P, long long r, int i, RfSegRows& S)\n{\n";
+        for (auto& h : row_loads_) o << "    S." << h[1] << "[i] = rf_ld<" << h[0] << ">(" << h[2] << ", r);\n";
+        o << "    (void)P; (void)r; (void)i; (void)S;\n}\n";
+        o << "RF_DEV void rf_seg_row(const RfParams& P, long long r, int i, const RfSegRows& S, RfAcc& A)\n{\n";
+        if (row_loads_.empty()) {
+            o << "    rf_row(P, r, A);\n    (void)i; (void)S;\n}\n\n";
+        } else {
+            o << "    rf_row_v(P, r, A";
+            for (auto& h : row_loads_) o << ", S." << h[1] << "[i]";
+            o << ");\n}\n\n";
+        }
+        o << "RF_DEV void rf_fold(const RfParams& P, long long run, RfAcc& A)\n{\n"
+             "    rf_ld_words(&A, (const RfAcc*)P.aux5 + run, (int)sizeof(RfAcc));\n}\n\n";
+        plan_.kernels.push_back({"rf_seg_part", 256, 0, KernelSpec::SEGPART});
+        plan_.kernels.push_back({"rf_seg_reduce", T, 0, KernelSpec::SEGREDUCE});
+        plan_.kernels.push_back({"rf_seg_fix", 512, 0, KernelSpec::SEGFIX});
+    }
+
+    static size_t size_of_ctype(const std::string& t)
+    {
+        if (t == "int8_t" || t == "uint8_t") return 1;
+        if (t == "int16_t" || t == "uint16_t") return 2;
+        if (t == "int32_t" || t == "uint32_t" || t == "float") return 4;
+        return 8;
     }
 
     // the final state of a folded accumulator `SA`, as a struct value
@@ -3394,6 +3406,7 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
     int threads_;
     Plan plan_;
     std::map<const ExprNode*, int> input_index_;
+    std::vector<std::array<std::string, 3>> row_loads_;  // emit_row's column loads: type, name, pointer
 };
 
 }  // namespace

@@ -54,7 +54,7 @@ struct KernelSpec {
     std::string name;
     int threads = 256;
     size_t smem = 0;
-    enum Role { MAIN, RANGE, STOP, COUNT, SCAN, SCATTER, INIT, FINAL, SEGCOUNT, SEGSCAN, SEGREDUCE, IXCOUNT, IXINIT,
+    enum Role { MAIN, RANGE, STOP, COUNT, SCAN, SCATTER, INIT, FINAL, SEGCOUNT, SEGSCAN, SEGPART, SEGREDUCE, SEGFIX, IXCOUNT, IXINIT,
                 IXBUILD } role = MAIN;
 };
 
@@ -83,7 +83,7 @@ struct Plan {
     size_t out_size = 0;                // bytes of the value output (C layout)
     bool out_is_table = false;
     size_t acc_bytes = 0;               // bytes of one unit's partial (scan-reduce, segmented reduce)
-    int seg_chunk = 256;                // segmented reduce: rows per chunk
+    int seg_items = 0;                  // segmented reduce: rows and run ends of a tile
     int ixf_input = -1;                 // input whose index a run replaces by a filtered one (-1: none)
     int union_inputs[2] = {-1, -1};     // union merge: the two merged vectors (Func inputs)
     int hg_hot = 0;                     // hash group-by: hottest keys folded per warp (index 2x)

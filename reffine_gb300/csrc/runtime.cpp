@@ -2221,20 +2221,21 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     P.aux1 = p->d_ptrs + RF_MAX_COLS;
     P.aux2 = p->d_tiles;
     P.aux3 = p->d_res;
-    long long nruns = 0;
+    long long nruns = 0, seg_tiles = 0;
     if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
         rf_table* vt = args[pl.drive_input].table;
         nruns = vt->cols[0].nvals;
-        long long nrows = vt->cols[0].logical;
-        size_t wmax = (size_t)(nruns + (nrows + pl.seg_chunk - 1) / pl.seg_chunk + 2);
-        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(nruns + 2) * 8, s) ||
-            !grow((void**)&p->seg_tmp, &p->seg_tmp_cap, (size_t)(nruns / 2048 + 4) * 8, s) ||
-            !grow(&p->seg_part, &p->seg_part_cap, wmax * pl.acc_bytes, s)) {
+        const long long nrows = vt->cols[0].logical;
+        seg_tiles = (nruns + nrows + pl.seg_items - 1) / pl.seg_items;
+        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(seg_tiles + 1) * 8, s) ||
+            !grow(&p->seg_part, &p->seg_part_cap, (size_t)(nruns + seg_tiles + 1) * pl.acc_bytes, s)) {
             free_table_mem(t.get());
             return fail(ctx, RF_ERR_OOM, "segmented-reduce buffers");
         }
         P.aux4 = p->seg_woff;
         P.aux5 = p->seg_part;
+        P.aux_n0 = nrows;
+        P.aux_n1 = seg_tiles;
     }
     if (union_merge) {
         // paired-row counts of the first vector, scanned in place (nA + 1 entries)
@@ -2290,9 +2291,10 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
             continue;
         }
         int grid = units;
-        if (k.role == rfg::KernelSpec::SEGCOUNT || k.role == rfg::KernelSpec::SEGREDUCE ||
-            k.role == rfg::KernelSpec::INIT)
-            grid = ctx->sm_count * 8;
+        if (k.role == rfg::KernelSpec::SEGCOUNT || k.role == rfg::KernelSpec::INIT) grid = ctx->sm_count * 8;
+        if (k.role == rfg::KernelSpec::SEGPART) grid = (int)(seg_tiles / 8 + 1);  // a warp per tile boundary
+        if (k.role == rfg::KernelSpec::SEGREDUCE) grid = (int)std::max<long long>(seg_tiles, 1);
+        if (k.role == rfg::KernelSpec::SEGFIX) grid = 1;
         if (pl.kind == rfg::PlanKind::HASH_GROUP && k.role == rfg::KernelSpec::MAIN)
             grid = std::max(1, p->max_units * t_grid_share / 100);
         if (k.role == rfg::KernelSpec::RANGE || k.role == rfg::KernelSpec::SCAN) grid = 1;
