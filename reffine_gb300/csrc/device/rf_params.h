@@ -69,7 +69,11 @@ typedef struct RfParams {
     int flags;
     int unit0;                 // first unit of this launch (a launch runs units unit0 .. unit0+grid-1)
     int rsv_;
+    void* oc[RF_MAX_COLS];     // table outputs: column values
+    unsigned* ov[RF_MAX_COLS]; // table outputs: validity words (vectorised)
 } RfParams;
+
+#define RF_MAT_TILE 2048  // elements of a tile of the materialisation kernels
 
 #define RF_EMPTY_KEY ((long long)0x8000000000000000ULL)
 

@@ -347,13 +347,18 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
 // finalize_vector, vinstr.h:113-135).
 //   The fragment defines rf_cond(P, r) (the iteration condition of element r) and
 //   rf_emit(P, r, o) (computes the element's iterators and outputs, writes them at output row o).
-//   Output columns: ((void**)P.aux0)[c]; validity words: ((unsigned**)P.aux1)[c];
-//   per-tile counts / offsets: (long long*)P.aux2; results (long long*)P.aux3:
-//   [0] = rows written, [1] = null count.
-//   Compaction (vectorize off) keeps passing elements in loop order: count per tile, one
-//   exclusive scan over tiles, then a scatter that ranks elements inside each tile with warp
-//   ballots.  Vectorised (on): every visited element is written; its condition becomes the
-//   validity bit.
+//   Output columns: P.oc[c]; validity words: P.ov[c]; a bit per element that passes, 32 elements
+//   from P.row_lo on to a word: (unsigned*)P.aux1; per-tile counts / offsets: (long long*)P.aux2;
+//   results (long long*)P.aux3: [0] = rows written, [1] = null count.
+//   Compaction (vectorize off) keeps passing elements in loop order: rf_count evaluates the
+//   condition once, writes its bits and each tile's count, and its last block turns the counts
+//   into offsets; rf_scatter lists a tile's passing elements in shared memory and emits them 256
+//   at a time, so every lane works and the output is written in order whatever share passes.
+//   Vectorised (on): every visited element is written; its condition becomes the validity bit.
+//   Both are bound by memory: a tile is RF_MAT_TILE elements and a block takes one tile at a time,
+//   so that eight blocks an SM keep loads in flight through the few barriers of a tile.  (One
+//   8192-element tile per SM with three barriers every 256 elements took 88 us to count and
+//   945 us to scatter 37 % of 20M rows of 24 bytes.)
 // ---------------------------------------------------------------------------------------
 #ifdef RF_MATERIALIZE
 RF_DEV void rf_mat_bounds(const RfParams& P, long long& lo, long long& hi)
@@ -369,9 +374,10 @@ RF_DEV void rf_mat_bounds(const RfParams& P, long long& lo, long long& hi)
 
 RF_DEV long long rf_mat_ntiles(const RfParams& P)
 {
-    return (P.row_hi - P.row_lo + P.tile_rows - 1) / P.tile_rows;
+    return (P.row_hi - P.row_lo + RF_MAT_TILE - 1) / RF_MAT_TILE;
 }
 
+// sum of v over the block, in every thread (sh: T / 32 words; ends with a barrier)
 template <int T>
 RF_DEV int rf_block_sum_int(int v, int* sh)
 {
@@ -380,105 +386,124 @@ RF_DEV int rf_block_sum_int(int v, int* sh)
     if (lane == 0) sh[warp] = v;
     __syncthreads();
     int t = 0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < T / 32; w++) t += sh[w];
+#pragma unroll
+    for (int w = 0; w < T / 32; w++) t += sh[w];
     __syncthreads();
     return t;
+}
+
+// exclusive scan of n tile counts in place by one block; total -> *total
+template <int T>
+RF_DEV void rf_mat_scan(long long* cnt, long long n, long long* total)
+{
+    constexpr int K = 8;  // counts a thread scans in its registers per step
+    __shared__ long long wsum[T / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long carry = 0;
+    for (long long base = 0; base < n; base += (long long)T * K) {
+        const long long i0 = base + (long long)threadIdx.x * K;
+        long long v[K], x = 0;
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = i0 + k < n ? __ldcg(cnt + i0 + k) : 0;
+#pragma unroll
+        for (int k = 0; k < K; k++) x += v[k];
+        long long incl = x;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        long long before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < T / 32; w++) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        long long o = carry + before + incl - x;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if (i0 + k < n) cnt[i0 + k] = o;
+            o += v[k];
+        }
+        carry += all;
+        __syncthreads();  // wsum is rewritten by the next step
+    }
+    if (threadIdx.x == 0) *total = carry;
 }
 
 template <int T>
 RF_DEV void rf_mat_count(const RfParams& P)
 {
     __shared__ int sh[T / 32];
+    __shared__ int last;
     long long lo, hi;
     rf_mat_bounds(P, lo, hi);
     long long* cnt = (long long*)P.aux2;
+    unsigned* bits = (unsigned*)P.aux1;
     const long long nt = rf_mat_ntiles(P);
+    const int lane = threadIdx.x & 31;
     for (long long tile = blockIdx.x; tile < nt; tile += gridDim.x) {
-        long long r0 = P.row_lo + tile * P.tile_rows, r1 = r0 + P.tile_rows;
-        if (r1 > hi) r1 = hi;
-        if (r0 < lo) r0 = lo;
+        const long long t0 = tile * RF_MAT_TILE;  // relative to row_lo, a multiple of 32
         int c = 0;
-        for (long long r = r0 + threadIdx.x; r < r1; r += T) c += rf_cond(P, r) ? 1 : 0;
-        int t = rf_block_sum_int<T>(c, sh);
-        if (threadIdx.x == 0) cnt[tile] = t;
-    }
-}
-
-// exclusive scan of the tile counts in place (one block); total -> aux3[0]
-RF_DEV void rf_mat_scan(const RfParams& P)
-{
-    __shared__ long long wsum[32];
-    __shared__ long long carry;
-    long long* cnt = (long long*)P.aux2;
-    const long long nt = rf_mat_ntiles(P);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (long long base = 0; base < nt; base += blockDim.x) {
-        long long i = base + threadIdx.x;
-        long long v = i < nt ? cnt[i] : 0;
-        long long x = v;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            long long y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        if (lane == 31) wsum[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            long long w = lane < nw ? wsum[lane] : 0;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                long long y = __shfl_up_sync(0xffffffffu, w, off);
-                if (lane >= off) w += y;
+        for (int j = 0; j < RF_MAT_TILE; j += T) {
+            const long long r = P.row_lo + t0 + j + threadIdx.x;
+            const unsigned m = __ballot_sync(0xffffffffu, r >= lo && r < hi && rf_cond(P, r));
+            if (lane == 0) {
+                bits[(t0 + j + threadIdx.x) >> 5] = m;
+                c += __popc(m);
             }
-            if (lane < nw) wsum[lane] = w;
         }
-        __syncthreads();
-        long long excl = carry + (warp ? wsum[warp - 1] : 0) + x - v;
-        if (i < nt) cnt[i] = excl;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += wsum[nw - 1];
-        __syncthreads();
+        c = rf_block_sum_int<T>(c, sh);
+        if (threadIdx.x == 0) __stcg(cnt + tile, (long long)c);
     }
-    if (threadIdx.x == 0) ((long long*)P.aux3)[0] = carry;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(P.counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    rf_mat_scan<T>(cnt, nt, (long long*)P.aux3);
+    if (threadIdx.x == 0) *P.counter = 0u;
 }
 
 template <int T>
 RF_DEV void rf_mat_scatter(const RfParams& P)
 {
-    __shared__ int wcnt[T / 32];
-    __shared__ int woff[T / 32 + 1];
-    long long lo, hi;
-    rf_mat_bounds(P, lo, hi);
+    constexpr int NW = RF_MAT_TILE / 32;  // words of a tile
+    static_assert(NW == 64, "a warp scans a tile's words two to a lane");
+    __shared__ unsigned short idx[RF_MAT_TILE];
     const long long* off = (const long long*)P.aux2;
+    const unsigned* bits = (const unsigned*)P.aux1;
     const long long nt = rf_mat_ntiles(P);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (long long tile = blockIdx.x; tile < nt; tile += gridDim.x) {
-        long long r0 = P.row_lo + tile * P.tile_rows, r1 = r0 + P.tile_rows;
-        if (r1 > hi) r1 = hi;
-        if (r0 < lo) r0 = lo;
-        long long base = off[tile];
-        for (long long c0 = r0; c0 < r1; c0 += T) {
-            long long r = c0 + threadIdx.x;
-            bool c = r < r1 && rf_cond(P, r);
-            unsigned m = __ballot_sync(0xffffffffu, c);
-            if (lane == 0) wcnt[warp] = __popc(m);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int s = 0;
-                for (int w = 0; w < T / 32; w++) {
-                    woff[w] = s;
-                    s += wcnt[w];
-                }
-                woff[T / 32] = s;
-            }
-            __syncthreads();
-            if (c) rf_emit(P, r, base + woff[warp] + __popc(m & ((1u << lane) - 1u)));
-            base += woff[T / 32];
-            __syncthreads();
+        const long long base = __ldg(off + tile);
+        // every warp scans the counts of all words, then lists its own share of them
+        const unsigned a = __ldg(bits + tile * NW + 2 * lane), b = __ldg(bits + tile * NW + 2 * lane + 1);
+        const int pa = __popc(a), pb = __popc(b);
+        int incl = pa + pb;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
         }
+        const int n = __shfl_sync(0xffffffffu, incl, 31);
+        const int ea = incl - pa - pb;
+#pragma unroll
+        for (int k = 0; k < NW / (T / 32); k++) {
+            const int w = warp * (NW / (T / 32)) + k;
+            const unsigned m = __shfl_sync(0xffffffffu, (w & 1) ? b : a, w >> 1);
+            const int o = __shfl_sync(0xffffffffu, (w & 1) ? ea + pa : ea, w >> 1);
+            if ((m >> lane) & 1u) idx[o + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(w * 32 + lane);
+        }
+        __syncthreads();
+        const long long r0 = P.row_lo + tile * RF_MAT_TILE;
+        for (int i = threadIdx.x; i < n; i += T) rf_emit(P, r0 + idx[i], base + i);
+        __syncthreads();  // the list is rewritten by the next tile
     }
 }
 
@@ -489,28 +514,31 @@ RF_DEV void rf_mat_write_all(const RfParams& P, int ncols)
     rf_mat_bounds(P, lo, hi);
     const long long nt = rf_mat_ntiles(P);
     const int lane = threadIdx.x & 31;
+    // the output starts at lo: where that is a whole number of words into the tiles, a warp's 32
+    // elements are one word of their own, else they share two words with the neighbouring warps
+    const bool whole = ((lo - P.row_lo) & 31) == 0;
     long long nulls = 0;
     for (long long tile = blockIdx.x; tile < nt; tile += gridDim.x) {
-        long long r0 = P.row_lo + tile * P.tile_rows, r1 = r0 + P.tile_rows;
-        if (r1 > hi) r1 = hi;
-        if (r0 < lo) r0 = lo;
-        for (long long c0 = r0; c0 < r1; c0 += T) {
-            long long r = c0 + threadIdx.x;
-            bool in = r < r1;
-            bool c = in && rf_cond(P, r);
+#pragma unroll
+        for (int j = 0; j < RF_MAT_TILE; j += T) {
+            const long long r = P.row_lo + tile * RF_MAT_TILE + j + threadIdx.x;
+            const bool in = r >= lo && r < hi;
+            const bool c = in && rf_cond(P, r);
             if (in) rf_emit(P, r, r - lo);
-            unsigned m = __ballot_sync(0xffffffffu, c);
-            unsigned act = __ballot_sync(0xffffffffu, in);
-            nulls += (lane == 0) ? __popc(act & ~m) : 0;
-            // lanes of a warp hold consecutive elements: their bits land in at most two words
-            long long o0 = __shfl_sync(0xffffffffu, r - lo, 0);
-            if (lane == 0 && act) {
-                long long w = o0 >> 5;
-                int sft = (int)(o0 & 31);
-                for (int col = 0; col < ncols; col++) {
-                    unsigned* bm = ((unsigned**)P.aux1)[col];
-                    atomicOr(bm + w, m << sft);
-                    if (sft && (m >> (32 - sft))) atomicOr(bm + w + 1, m >> (32 - sft));
+            const unsigned m = __ballot_sync(0xffffffffu, c);
+            const unsigned act = __ballot_sync(0xffffffffu, in);
+            nulls += __popc(act & ~m);
+            if (!act) continue;
+            const int f = __ffs(act) - 1;  // the warp's first element in range
+            const long long o0 = __shfl_sync(0xffffffffu, r - lo, f);
+            for (int col = lane; col < ncols; col += 32) {
+                unsigned* bm = P.ov[col] + (o0 >> 5);
+                if (whole) {
+                    *bm = m;
+                } else {
+                    const int sft = (int)(o0 & 31);
+                    atomicOr(bm, (m >> f) << sft);
+                    if (sft && ((m >> f) >> (32 - sft))) atomicOr(bm + 1, (m >> f) >> (32 - sft));
                 }
             }
         }
@@ -522,10 +550,6 @@ RF_DEV void rf_mat_write_all(const RfParams& P, int ncols)
     extern "C" __global__ void __launch_bounds__(T) rf_count(const __grid_constant__ RfParams P)         \
     {                                                                                                    \
         rf_mat_count<T>(P);                                                                              \
-    }                                                                                                    \
-    extern "C" __global__ void __launch_bounds__(1024) rf_scan(const __grid_constant__ RfParams P)      \
-    {                                                                                                    \
-        rf_mat_scan(P);                                                                                  \
     }                                                                                                    \
     extern "C" __global__ void __launch_bounds__(T) rf_scatter(const __grid_constant__ RfParams P)       \
     {                                                                                                    \

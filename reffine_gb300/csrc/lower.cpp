@@ -11,6 +11,8 @@
 //   expressions        src/pass/cemitter.cpp:112-160 (C++ operators and std::max/std::min)
 #include "lower.h"
 
+#include "device/rf_params.h"
+
 #include <algorithm>
 #include <array>
 #include <cstdio>
@@ -277,6 +279,7 @@ public:
         if (root->type.is_vector()) {
             if (root->kind != NodeKind::OP) throw LowerError("a vector output must be an Op");
             lower_op(root);
+            plan_.tile_rows = RF_MAT_TILE;
         } else {
             std::vector<const Reduce*> reds;
             find_reduces(fn_->output, reds);
@@ -2840,9 +2843,9 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             elem(E, body);
             std::ostringstream w;
             size_t c = 0;
-            w << "    ((int64_t*)((void* const*)P.aux0)[" << c++ << "])[o] = it;\n";
+            w << "    ((int64_t*)P.oc[" << c++ << "])[o] = it;\n";
             for (auto& x : op.outputs) {
-                w << "    ((" << ctype(x->type) << "*)((void* const*)P.aux0)[" << c << "])[o] = (" << ctype(x->type) << ")("
+                w << "    ((" << ctype(x->type) << "*)P.oc[" << c << "])[o] = (" << ctype(x->type) << ")("
                   << E.ev(x).c << ");\n";
                 c++;
             }
@@ -2862,7 +2865,6 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             plan_.kernels.push_back({"rf_hg_agg", HT, smem, KernelSpec::MAIN});
         }
         plan_.kernels.push_back({"rf_count", T, 0, KernelSpec::COUNT});
-        plan_.kernels.push_back({"rf_scan", 1024, 0, KernelSpec::SCAN});
         plan_.kernels.push_back({"rf_scatter", T, 0, KernelSpec::SCATTER});
         plan_.aggs = L;
         plan_.device_range = false;
@@ -2965,9 +2967,9 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             body_of(E, b);
             std::ostringstream w;
             size_t c = 0;
-            w << "    ((" << Ty << "*)((void* const*)P.aux0)[" << c++ << "])[o] = it;\n";
+            w << "    ((" << Ty << "*)P.oc[" << c++ << "])[o] = it;\n";
             for (auto& x : op.outputs) {
-                w << "    ((" << ctype(x->type) << "*)((void* const*)P.aux0)[" << c << "])[o] = (" << ctype(x->type) << ")("
+                w << "    ((" << ctype(x->type) << "*)P.oc[" << c << "])[o] = (" << ctype(x->type) << ")("
                   << E.ev(x).c << ");\n";
                 c++;
             }
@@ -2981,7 +2983,6 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             plan_.kernels.push_back({"rf_write_all", T, 0, KernelSpec::FINAL});
         } else {
             plan_.kernels.push_back({"rf_count", T, 0, KernelSpec::COUNT});
-            plan_.kernels.push_back({"rf_scan", 1024, 0, KernelSpec::SCAN});
             plan_.kernels.push_back({"rf_scatter", T, 0, KernelSpec::SCATTER});
         }
         plan_.source = o.str();
@@ -3075,9 +3076,9 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
         E.bind(op.iters[0], E.scalar("it", it->type));
         std::ostringstream w;
         size_t c = 0;
-        w << "    ((" << ctype(it->type) << "*)((void* const*)P.aux0)[" << c++ << "])[o] = it;\n";
+        w << "    ((" << ctype(it->type) << "*)P.oc[" << c++ << "])[o] = it;\n";
         for (auto& x : op.outputs) {
-            w << "    ((" << ctype(x->type) << "*)((void* const*)P.aux0)[" << c << "])[o] = (" << ctype(x->type) << ")("
+            w << "    ((" << ctype(x->type) << "*)P.oc[" << c << "])[o] = (" << ctype(x->type) << ")("
               << E.ev(x).c << ");\n";
             c++;
         }
@@ -3107,7 +3108,7 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             o << "        const bool ok = (li < nA && rf_valid(" << A << ".valid, li)) || (ri < nB && rf_valid(" << B
               << ".valid, ri));\n";
             o << "        if (ok)\n            for (int col = 0; col < " << plan_.out_cols.size()
-              << "; col++) atomicOr(((unsigned**)P.aux1)[col] + (pos >> 5), 1u << (pos & 31));\n";
+              << "; col++) atomicOr(P.ov[col] + (pos >> 5), 1u << (pos & 31));\n";
             o << "        else\n            nulls++;\n";
         }
         o << "    }\n";
@@ -3247,12 +3248,12 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             std::ostringstream w;
             size_t c = 0;
             for (auto& i : op.iters) {
-                w << "    ((" << ctype(i->type) << "*)((void* const*)P.aux0)[" << c << "])[o] = (" << ctype(i->type)
+                w << "    ((" << ctype(i->type) << "*)P.oc[" << c << "])[o] = (" << ctype(i->type)
                   << ")(" << E.ev(i).c << ");\n";
                 c++;
             }
             for (auto& x : op.outputs) {
-                w << "    ((" << ctype(x->type) << "*)((void* const*)P.aux0)[" << c << "])[o] = (" << ctype(x->type)
+                w << "    ((" << ctype(x->type) << "*)P.oc[" << c << "])[o] = (" << ctype(x->type)
                   << ")(" << E.ev(x).c << ");\n";
                 c++;
             }
@@ -3266,7 +3267,6 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             plan_.kernels.push_back({"rf_write_all", T, 0, KernelSpec::FINAL});
         } else {
             plan_.kernels.push_back({"rf_count", T, 0, KernelSpec::COUNT});
-            plan_.kernels.push_back({"rf_scan", 1024, 0, KernelSpec::SCAN});
             plan_.kernels.push_back({"rf_scatter", T, 0, KernelSpec::SCATTER});
         }
         plan_.source = src.str();
@@ -3376,12 +3376,12 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             std::ostringstream w;
             size_t c = 0;
             for (auto& i : op.iters) {
-                w << "    ((" << ctype(i->type) << "*)((void* const*)P.aux0)[" << c << "])[o] = (" << ctype(i->type)
+                w << "    ((" << ctype(i->type) << "*)P.oc[" << c << "])[o] = (" << ctype(i->type)
                   << ")(" << E.ev(i).c << ");\n";
                 c++;
             }
             for (auto& o : op.outputs) {
-                w << "    ((" << ctype(o->type) << "*)((void* const*)P.aux0)[" << c << "])[o] = (" << ctype(o->type)
+                w << "    ((" << ctype(o->type) << "*)P.oc[" << c << "])[o] = (" << ctype(o->type)
                   << ")(" << E.ev(o).c << ");\n";
                 c++;
             }
@@ -3395,7 +3395,6 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             plan_.kernels.push_back({"rf_write_all", T, 0, KernelSpec::FINAL});
         } else {
             plan_.kernels.push_back({"rf_count", T, 0, KernelSpec::COUNT});
-            plan_.kernels.push_back({"rf_scan", 1024, 0, KernelSpec::SCAN});
             plan_.kernels.push_back({"rf_scatter", T, 0, KernelSpec::SCATTER});
         }
         plan_.source = src.str();

@@ -54,8 +54,8 @@ struct KernelSpec {
     std::string name;
     int threads = 256;
     size_t smem = 0;
-    enum Role { MAIN, RANGE, STOP, COUNT, SCAN, SCATTER, INIT, FINAL, SEGCOUNT, SEGSCAN, SEGPART, SEGREDUCE, SEGFIX, IXCOUNT, IXINIT,
-                IXBUILD } role = MAIN;
+    enum Role { MAIN, RANGE, STOP, COUNT, SCATTER, INIT, FINAL, SEGCOUNT, SEGSCAN, SEGPART, SEGREDUCE, SEGFIX, IXCOUNT,
+                IXINIT, IXBUILD } role = MAIN;
 };
 
 struct Plan {

@@ -180,8 +180,7 @@ struct rf_plan {
     size_t batch_smem = 0;
     int batch_threads = 0;
     // table outputs
-    void** d_ptrs = nullptr;          // device array: output column pointers, then bitmap pointers
-    long long* d_tiles = nullptr;     // per-tile counts / offsets
+    long long* d_tiles = nullptr;     // a bit per element, then per-tile counts / offsets
     size_t tiles_cap = 0;             // bytes
     long long* d_res = nullptr;       // [rows written, null count]
     // hash group-by

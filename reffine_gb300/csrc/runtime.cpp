@@ -1091,13 +1091,13 @@ int build_plan(rf_ctx* ctx, const std::shared_ptr<reffine::Func>& fn, bool vecto
     // the plan's own device buffers, carved from one allocation of the context's stream-ordered
     // pool (compiling many plans costs no device-wide synchronisation):
     //   [partials of the units][completion counter 64 B][loop range 64 B][value result]
-    //   [table outputs: column pointer array][results 64 B]
+    //   [table outputs: results 64 B]
     p->partials_bytes = (size_t)p->reduce_units * (p->plan.acc_bytes ? p->plan.acc_bytes : 8);
     const size_t osz = p->plan.out_size ? p->plan.out_size : 8;
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
     const size_t o_counter = al(p->partials_bytes), o_range = o_counter + 256, o_out = o_range + 256;
-    const size_t o_ptrs = o_out + al(osz), o_res = o_ptrs + al(sizeof(void*) * 2 * RF_MAX_COLS);
-    const size_t total = p->plan.out_is_table ? o_res + 256 : o_ptrs;
+    const size_t o_res = o_out + al(osz);
+    const size_t total = p->plan.out_is_table ? o_res + 256 : o_res;
     unsigned char* base = nullptr;
     CUDA_TRY(ctx, pool_alloc((void**)&base, total, ctx->stream));
     p->buf = base;
@@ -1105,10 +1105,7 @@ int build_plan(rf_ctx* ctx, const std::shared_ptr<reffine::Func>& fn, bool vecto
     p->counter = (unsigned*)(base + o_counter);
     p->range = (long long*)(base + o_range);
     p->dout = base + o_out;
-    if (p->plan.out_is_table) {
-        p->d_ptrs = (void**)(base + o_ptrs);
-        p->d_res = (long long*)(base + o_res);
-    }
+    if (p->plan.out_is_table) p->d_res = (long long*)(base + o_res);
     CUDA_TRY(ctx, cudaMemsetAsync(p->counter, 0, 64, ctx->stream));
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));  // ready for use on any stream
     return RF_OK;
@@ -1494,7 +1491,6 @@ int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, RfParams
         int grid = 1;
         switch (k.role) {
             case rfg::KernelSpec::RANGE: grid = 1; break;
-            case rfg::KernelSpec::SCAN: grid = 1; break;
             case rfg::KernelSpec::STOP: grid = (int)std::min<long long>(std::max<long long>((hi - lo + 255) / 256, 1), ctx->sm_count * 8); break;
             case rfg::KernelSpec::MAIN: grid = units; break;
             default: grid = units; break;
@@ -2170,7 +2166,6 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     t->name = "out";
     t->cols.resize(nc);
     t->present.assign(nc, 1);
-    std::vector<void*> hptrs(2 * RF_MAX_COLS, nullptr);
     // output columns of `rows` rows (validity bitmaps when vectorised)
     auto alloc_cols = [&](long long rows) -> int {
         for (size_t c = 0; c < nc; c++) {
@@ -2183,20 +2178,19 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
                 return fail(ctx, RF_ERR_OOM, "output column allocation (%zu bytes) failed", bytes);
             dc.data_cap = bytes;
             dc.data = dc.data_buf;
-            hptrs[c] = dc.data_buf;
+            P.oc[c] = dc.data_buf;
             if (pl.vectorize) {
                 size_t vb = (size_t)((std::max<long long>(rows, 1) + 31) / 32) * 4;
                 if (pool_alloc(&dc.valid_buf, vb + 16, s) != cudaSuccess)
                     return fail(ctx, RF_ERR_OOM, "output bitmap allocation failed");
                 dc.valid_cap = vb;
                 CUDA_TRY(ctx, cudaMemsetAsync(dc.valid_buf, 0, vb + 16, s));
-                hptrs[RF_MAX_COLS + c] = dc.valid_buf;
+                P.ov[c] = (unsigned*)dc.valid_buf;
             }
         }
-        CUDA_TRY(ctx, cudaMemcpyAsync(p->d_ptrs, hptrs.data(), sizeof(void*) * hptrs.size(), cudaMemcpyHostToDevice, s));
         return RF_OK;
     };
-    // A compacting materialisation (count, scan, scatter) learns its row count from the scan: the
+    // A compacting materialisation (count, scatter) learns its row count from the count: the
     // columns are then allocated at exactly that size before the scatter, so an output holds its
     // rows, not the loop's range (a hash group-by's slot table is ~2.2x the distinct keys).  A
     // vectorised one writes every visited element and is allocated at the range up front.
@@ -2210,16 +2204,15 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         return rc;
     }
     long long ntiles = (hi - lo + P.tile_rows - 1) / P.tile_rows;
-    if ((size_t)std::max<long long>(ntiles, 1) * 8 > p->tiles_cap) {  // tiles_cap: bytes
-        if (!grow((void**)&p->d_tiles, &p->tiles_cap, (size_t)std::max<long long>(ntiles, 1024) * 8, s)) {
-            free_table_mem(t.get());
-            return fail(ctx, RF_ERR_OOM, "tile buffer allocation failed");
-        }
+    // [a bit per element, whole tiles][count / offset of each tile]
+    const size_t bit_bytes = (size_t)std::max<long long>(ntiles, 1) * (RF_MAT_TILE / 8);
+    if (!grow((void**)&p->d_tiles, &p->tiles_cap, bit_bytes + (size_t)std::max<long long>(ntiles, 1) * 8, s)) {
+        free_table_mem(t.get());
+        return fail(ctx, RF_ERR_OOM, "tile buffer allocation failed");
     }
     CUDA_TRY(ctx, cudaMemsetAsync(p->d_res, 0, 64, s));
-    P.aux0 = p->d_ptrs;
-    P.aux1 = p->d_ptrs + RF_MAX_COLS;
-    P.aux2 = p->d_tiles;
+    P.aux1 = p->d_tiles;
+    P.aux2 = (unsigned char*)p->d_tiles + bit_bytes;
     P.aux3 = p->d_res;
     long long nruns = 0, seg_tiles = 0;
     if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
@@ -2297,7 +2290,10 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         if (k.role == rfg::KernelSpec::SEGFIX) grid = 1;
         if (pl.kind == rfg::PlanKind::HASH_GROUP && k.role == rfg::KernelSpec::MAIN)
             grid = std::max(1, p->max_units * t_grid_share / 100);
-        if (k.role == rfg::KernelSpec::RANGE || k.role == rfg::KernelSpec::SCAN) grid = 1;
+        // the materialisation kernels take a tile a block, as many blocks as fill the GPU four times
+        if (k.role == rfg::KernelSpec::COUNT || k.role == rfg::KernelSpec::FINAL || (int)i == iscatter)
+            grid = (int)std::min<long long>(std::max<long long>(ntiles, 1), ctx->sm_count * 32);
+        if (k.role == rfg::KernelSpec::RANGE) grid = 1;
         if (k.role == rfg::KernelSpec::STOP)
             grid = (int)std::min<long long>(std::max<long long>((hi - lo + 255) / 256, 1), ctx->sm_count * 8);
         if ((rc = launch(ctx, p->fns[i], grid, k.threads, k.smem, s, &P))) {

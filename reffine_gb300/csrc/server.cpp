@@ -80,7 +80,7 @@ size_t footprint_of(rf_plan* p, long long lo, long long hi)
     }
     size_t row_bytes = 8;
     for (auto& c : pl.out_cols) row_bytes += c.size();
-    size_t bytes = (size_t)rows * row_bytes + (size_t)(rows / pl.tile_rows + 2) * 8;
+    size_t bytes = (size_t)rows * row_bytes + (size_t)(rows / pl.tile_rows + 2) * (8 + RF_MAT_TILE / 8);
     if (pl.kind == rfg::PlanKind::HASH_GROUP) bytes += (size_t)rows * 2 * (8 + pl.acc_bytes);
     return bytes;
 }
