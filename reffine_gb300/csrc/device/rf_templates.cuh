@@ -343,10 +343,122 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
 
 
 // ---------------------------------------------------------------------------------------
+// Merge co-iteration of sorted key columns (InterSpace and UnionSpace, iter_space.cpp:217-364).
+// A row's partner in another vector is the row (first row of the key there) + (the row's rank among
+// its own vector's equal keys), as the two-pointer walk pairs duplicates.  Rows are taken in tiles
+// of RF_MAT_TILE: rf_merge_bound finds, a warp to a tile, where the other vector's rows of the
+// tile's keys begin (they end where the next tile's begin), and rf_merge_walk copies the tile's keys
+// and that window into shared memory, where a thread searches once for its first row and walks on
+// for the others.  A window larger than the buffer is searched in place.  The keys are so read
+// once; the walk's shared-memory latency is covered by the other blocks of the SM.  (Two binary
+// searches of the whole columns a row, in each of two kernels: 3.8 ms for 5M rows against 4M.)
+// Keys out of order give other partners, never an access outside the columns.
+// ---------------------------------------------------------------------------------------
+#ifdef RF_MERGE
+#define RF_MERGE_CAP 3584  // window keys of 8 bytes held (28 KiB beside the tile's 16 KiB)
+
+template <class K>
+RF_DEV K rf_key(const RfCol& c, long long i)
+{
+    return RfLd<K>::ldg(c.data, i);
+}
+
+// (whole warp) the rank of row x of `a` among the equal keys from row `lo` on
+template <class K>
+RF_DEV long long rf_merge_rank(const RfCol& a, long long lo, long long x, K key)
+{
+    if (x <= lo || rf_key<K>(a, x - 1) != key) return 0;
+    return x - rf_warp_search(lo, x, [&](long long i) { return rf_key<K>(a, i) < key; });
+}
+
+// (whole warp) first row of `b` from row `lo` on whose key is not below `key`
+template <class K>
+RF_DEV long long rf_merge_bound(const RfCol& b, long long lo, K key)
+{
+    return rf_warp_search(lo, b.len, [&](long long i) { return rf_key<K>(b, i) < key; });
+}
+
+template <class K>
+struct RfMergeBuf {
+    K key[RF_MAT_TILE];
+    long long win[RF_MERGE_CAP];  // the window's keys, then a value per row of the tile
+};
+
+// the tile's keys (n rows of `a` from row r0 on), for rf_merge_walk; the whole block
+template <int T, class K>
+RF_DEV void rf_merge_load(RfMergeBuf<K>& B, const RfCol& a, long long r0, int n)
+{
+    for (int i = threadIdx.x; i < n; i += T) B.key[i] = rf_key<K>(a, r0 + i);
+}
+
+// The thread's RF_MAT_TILE / T consecutive rows of the tile (from row `from` on): for the j-th,
+// f(j, row, key, first row of b at or above the key, rank).  rank0: the rank of the tile's first
+// row; w0, w1: the window.  The whole block; ends with a barrier, after which B.win is free.
+template <int T, class K, class F>
+RF_DEV void rf_merge_walk(RfMergeBuf<K>& B, long long r0, int n, long long from, long long rank0, const RfCol& b,
+                          long long w0, long long w1, F f)
+{
+    constexpr int R = RF_MAT_TILE / T, CAP = RF_MERGE_CAP * 8 / (int)sizeof(K);
+    if (w0 < 0) w0 = 0;
+    if (w1 > b.len) w1 = b.len;
+    const long long wn = w1 > w0 ? w1 - w0 : 0;
+    const bool held = wn <= CAP;
+    K* win = (K*)B.win;
+    if (held)
+        for (int i = threadIdx.x; i < (int)wn; i += T) win[i] = rf_key<K>(b, w0 + i);
+    __syncthreads();
+    auto at = [&](long long i) { return held ? win[i] : rf_key<K>(b, w0 + i); };
+    const int beg = from > r0 ? (from - r0 < n ? (int)(from - r0) : n) : 0;
+    const int i0 = (int)threadIdx.x * R;
+    long long p = 0, rank = 0;
+    K prev = K(0);
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const int i = i0 + j;
+        if (i < beg || i >= n) continue;
+        const K key = B.key[i];
+        if (any && key == prev) {
+            rank++;
+        } else {
+            long long lo = p, hi = wn;
+            rank = 0;
+            if (any) {
+                // the next key's rows are close by in most tables: a few steps, then a search
+                for (int k = 0; k < 4 && lo < hi && at(lo) < key; k++) lo++;
+                if (!(lo < hi && at(lo) < key)) hi = lo;
+            } else if (i > beg && B.key[i - 1] == key) {
+                int l = beg, h = i - 1;  // the first row of the key in the tile
+                while (l < h) {
+                    const int m = (l + h) >> 1;
+                    if (B.key[m] < key) l = m + 1;
+                    else h = m;
+                }
+                rank = i - l + (l == 0 ? rank0 : 0);
+            } else if (i == 0) {
+                rank = rank0;
+            }
+            while (lo < hi) {
+                const long long m = (lo + hi) >> 1;
+                if (at(m) < key) lo = m + 1;
+                else hi = m;
+            }
+            p = lo;
+        }
+        any = true;
+        prev = key;
+        f(j, r0 + i, key, w0 + p, rank);
+    }
+    __syncthreads();
+}
+#endif  // RF_MERGE
+
+// ---------------------------------------------------------------------------------------
 // Template 3: Op materialisation (LoopGen::visit(Op), loopgen.cpp:113-204, and
 // finalize_vector, vinstr.h:113-135).
 //   The fragment defines rf_cond(P, r) (the iteration condition of element r) and
-//   rf_emit(P, r, o) (computes the element's iterators and outputs, writes them at output row o).
+//   rf_emit(P, r, o) (computes the element's iterators and outputs, writes them at output row o),
+//   and with RF_MAT_PREP rf_mat_prep<T>(P, tile), which a block runs before the tile's conditions.
 //   Output columns: P.oc[c]; validity words: P.ov[c]; a bit per element that passes, 32 elements
 //   from P.row_lo on to a word: (unsigned*)P.aux1; per-tile counts / offsets: (long long*)P.aux2;
 //   results (long long*)P.aux3: [0] = rows written, [1] = null count.
@@ -433,6 +545,7 @@ RF_DEV void rf_mat_scan(long long* cnt, long long n, long long* total)
     if (threadIdx.x == 0) *total = carry;
 }
 
+#ifndef RF_UNION  // (a union writes its visits itself)
 template <int T>
 RF_DEV void rf_mat_count(const RfParams& P)
 {
@@ -447,6 +560,9 @@ RF_DEV void rf_mat_count(const RfParams& P)
     for (long long tile = blockIdx.x; tile < nt; tile += gridDim.x) {
         const long long t0 = tile * RF_MAT_TILE;  // relative to row_lo, a multiple of 32
         int c = 0;
+#ifdef RF_MAT_PREP
+        rf_mat_prep<T>(P, tile);
+#endif
 #pragma unroll
         for (int j = 0; j < RF_MAT_TILE; j += T) {
             const long long r = P.row_lo + t0 + j + threadIdx.x;
@@ -519,6 +635,9 @@ RF_DEV void rf_mat_write_all(const RfParams& P, int ncols)
     const bool whole = ((lo - P.row_lo) & 31) == 0;
     long long nulls = 0;
     for (long long tile = blockIdx.x; tile < nt; tile += gridDim.x) {
+#ifdef RF_MAT_PREP
+        rf_mat_prep<T>(P, tile);
+#endif
 #pragma unroll
         for (int j = 0; j < RF_MAT_TILE; j += T) {
             const long long r = P.row_lo + tile * RF_MAT_TILE + j + threadIdx.x;
@@ -559,7 +678,218 @@ RF_DEV void rf_mat_write_all(const RfParams& P, int ncols)
     {                                                                                                    \
         rf_mat_write_all<T>(P, NCOLS);                                                                   \
     }
+#endif  // RF_UNION
 #endif  // RF_MATERIALIZE
+
+// ---------------------------------------------------------------------------------------
+// Union merge of two sorted int64 key columns A and B (template 3's tiles over B, then over both).
+//   The fragment defines rf_u_a(P), rf_u_b(P) (the key columns), rf_u_write(P, li, ri, v, o) (the
+//   visit's outputs at output row o) and, vectorised, RF_UNION_VALID (output columns).
+//   (long long*)P.aux4: {rank, window start} of each tile boundary of A (P.aux_n0 tiles + 1), then of
+//   B (P.aux_n1 + 1); (long long*)P.aux5: of each B row, the A rows up to its key if it is unpaired,
+//   else -1; (unsigned*)P.aux1: a bit per B row, unpaired; (unsigned short*)P.aux0: unpaired rows of
+//   the tile before each word; (long long*)P.aux2: and of the tiles before each tile; P.aux3[0]: visits.
+// Both key columns are read twice (once to find what is unpaired, once to write); the rest of the
+// traffic is the outputs.  (3M rows against 2.5M with 40 % of the keys shared: 1728 us a call with
+// three binary searches a row in each of two kernels on one block an SM.)
+// ---------------------------------------------------------------------------------------
+#ifdef RF_UNION
+// the first row of c at or after lo with a key above `key`, knowing that row hi has one (or is the end)
+RF_DEV long long rf_u_upper(const RfCol& c, long long lo, long long hi, long long key)
+{
+    if (hi > c.len) hi = c.len;
+    while (lo < hi) {
+        const long long m = (lo + hi) >> 1;
+        if (rf_key<int64_t>(c, m) <= key) lo = m + 1;
+        else hi = m;
+    }
+    return lo;
+}
+
+// (whole warp) {rank, window start} of boundary t of the tiles of `a`
+RF_DEV void rf_u_bound(const RfCol& a, const RfCol& b, long long t, long long* out)
+{
+    const long long x = t * RF_MAT_TILE;
+    long long rank = 0, lb = b.len;
+    if (x < a.len) {
+        const long long key = rf_key<int64_t>(a, x);
+        rank = rf_merge_rank<int64_t>(a, 0, x, key);
+        lb = rf_merge_bound<int64_t>(b, 0, key);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        out[2 * t] = rank;
+        out[2 * t + 1] = lb;
+    }
+}
+
+RF_DEV void rf_u_part_all(const RfParams& P)
+{
+    const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    long long* out = (long long*)P.aux4;
+    if (w <= P.aux_n0) rf_u_bound(rf_u_a(P), rf_u_b(P), w, out);
+    else if (w - P.aux_n0 - 1 <= P.aux_n1) rf_u_bound(rf_u_b(P), rf_u_a(P), w - P.aux_n0 - 1, out + 2 * (P.aux_n0 + 1));
+}
+
+template <int T>
+RF_DEV void rf_u_count_all(const RfParams& P)
+{
+    constexpr int R = RF_MAT_TILE / T;
+    __shared__ RfMergeBuf<int64_t> B;
+    __shared__ int sh[T / 32];
+    __shared__ int last;
+    const RfCol &a = rf_u_a(P), &b = rf_u_b(P);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long* cnt = (long long*)P.aux2;
+    for (long long tile = blockIdx.x; tile < P.aux_n1; tile += gridDim.x) {
+        const long long r0 = tile * RF_MAT_TILE;
+        const int n = b.len - r0 < RF_MAT_TILE ? (int)(b.len - r0) : RF_MAT_TILE;
+        const long long* part = (const long long*)P.aux4 + 2 * (P.aux_n0 + 1) + 2 * tile;
+        rf_merge_load<T>(B, b, r0, n);
+        long long j[R];
+#pragma unroll
+        for (int q = 0; q < R; q++) j[q] = -1;
+        rf_merge_walk<T>(B, r0, n, 0, __ldg(part), a, __ldg(part + 1), __ldg(part + 3),
+                         [&](int q, long long, long long key, long long lb, long long rank) {
+                             const long long i = lb + rank;
+                             if (!(i < a.len && rf_key<int64_t>(a, i) == key)) j[q] = rf_u_upper(a, lb, i, key);
+                         });
+#pragma unroll
+        for (int q = 0; q < R; q++) B.win[(int)threadIdx.x * R + q] = j[q];
+        __syncthreads();
+        int c = 0;
+#pragma unroll
+        for (int q = 0; q < RF_MAT_TILE; q += T) {
+            const int i = q + (int)threadIdx.x;
+            const long long x = B.win[i];
+            if (i < n) ((long long*)P.aux5)[r0 + i] = x;
+            const unsigned m = __ballot_sync(0xffffffffu, x >= 0);
+            if (lane == 0) {
+                ((unsigned*)P.aux1)[(r0 + i) >> 5] = m;
+                B.key[i >> 5] = __popc(m);  // the keys are not read again
+                c += __popc(m);
+            }
+        }
+        c = rf_block_sum_int<T>(c, sh);
+        if (threadIdx.x == 0) __stcg(cnt + tile, (long long)c);
+        if (warp == 0) {  // words before each word, two words to a lane
+            const int x = (int)B.key[2 * lane], y = (int)B.key[2 * lane + 1];
+            int incl = x + y;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int z = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += z;
+            }
+            ((unsigned*)P.aux0)[tile * (RF_MAT_TILE / 64) + lane] = (unsigned)(incl - x - y) | (unsigned)(incl - y) << 16;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(P.counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    rf_mat_scan<T>(cnt, P.aux_n1, (long long*)P.aux3);
+    if (threadIdx.x == 0) {
+        ((long long*)P.aux3)[0] += a.len;
+        *P.counter = 0u;
+    }
+}
+
+// writes a visit; false: a null row.  Keys out of order (the walk needs sorted iterator columns) can
+// move a visit, never past the output: positions are checked against the visit count.
+RF_DEV bool rf_u_visit(const RfParams& P, long long li, long long ri, long long v, long long pos, long long V)
+{
+    if (pos < 0 || pos >= V) {
+        rf_set_err(P, RF_DEVERR_RANGE);
+        return true;
+    }
+    rf_u_write(P, li, ri, v, pos);
+#ifdef RF_UNION_VALID
+    const RfCol &a = rf_u_a(P), &b = rf_u_b(P);
+    if (!((li < a.len && rf_valid(a.valid, li)) || (ri < b.len && rf_valid(b.valid, ri)))) return false;
+    for (int col = 0; col < RF_UNION_VALID; col++) atomicOr(P.ov[col] + (pos >> 5), 1u << (pos & 31));
+#endif
+    return true;
+}
+
+template <int T>
+RF_DEV void rf_u_emit_all(const RfParams& P)
+{
+    constexpr int R = RF_MAT_TILE / T, NW = RF_MAT_TILE / 32;
+    __shared__ RfMergeBuf<int64_t> B;
+    const RfCol &a = rf_u_a(P), &b = rf_u_b(P);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long* off = (const long long*)P.aux2;
+    const unsigned* bits = (const unsigned*)P.aux1;
+    const unsigned short* before = (const unsigned short*)P.aux0;
+    const long long V = ((const long long*)P.aux3)[0];
+    long long nulls = 0;
+    for (long long tile = blockIdx.x; tile < P.aux_n0 + P.aux_n1; tile += gridDim.x) {
+        if (tile < P.aux_n0) {  // a tile of A: every row has a visit
+            const long long r0 = tile * RF_MAT_TILE;
+            const int n = a.len - r0 < RF_MAT_TILE ? (int)(a.len - r0) : RF_MAT_TILE;
+            const long long* part = (const long long*)P.aux4 + 2 * tile;
+            rf_merge_load<T>(B, a, r0, n);
+            long long l[R], x[R];
+#pragma unroll
+            for (int q = 0; q < R; q++) l[q] = x[q] = 0;
+            rf_merge_walk<T>(B, r0, n, 0, __ldg(part), b, __ldg(part + 1), __ldg(part + 3),
+                             [&](int q, long long, long long key, long long lb, long long rank) {
+                                 const long long i = lb + rank;
+                                 l[q] = lb;
+                                 x[q] = i < b.len && rf_key<int64_t>(b, i) == key ? i : rf_u_upper(b, lb, i, key);
+                             });
+#pragma unroll
+            for (int q = 0; q < R; q++) {
+                B.win[(int)threadIdx.x * R + q] = l[q];
+                B.key[(int)threadIdx.x * R + q] = x[q];
+            }
+            __syncthreads();
+            for (int i = threadIdx.x; i < n; i += T) {
+                const long long lb = B.win[i];
+                long long u = V - a.len;  // unpaired rows of B before its row lb
+                if (lb < b.len)
+                    u = __ldg(off + (lb / RF_MAT_TILE)) + __ldg(before + (lb >> 5)) +
+                        __popc(__ldg(bits + (lb >> 5)) & ((1u << (lb & 31)) - 1u));
+                nulls += !rf_u_visit(P, r0 + i, B.key[i], rf_key<int64_t>(a, r0 + i), r0 + i + u, V);
+            }
+        } else {  // a tile of B: its unpaired rows, listed in shared memory
+            const long long t = tile - P.aux_n0, r0 = t * RF_MAT_TILE, base = __ldg(off + t);
+            unsigned short* idx = (unsigned short*)B.win;
+            int total = 0;
+            for (int w = warp; w < NW; w += T / 32) {
+                const unsigned m = __ldg(bits + t * NW + w);
+                if ((m >> lane) & 1u)
+                    idx[__ldg(before + t * NW + w) + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(w * 32 + lane);
+            }
+            total = __ldg(before + t * NW + NW - 1) + __popc(__ldg(bits + t * NW + NW - 1));
+            __syncthreads();
+            for (int i = threadIdx.x; i < total; i += T) {
+                const long long j = r0 + idx[i], li = ((const long long*)P.aux5)[j];
+                nulls += !rf_u_visit(P, li, j, rf_key<int64_t>(b, j), li + base + i, V);
+            }
+        }
+        __syncthreads();
+    }
+    if (nulls) atomicAdd((unsigned long long*)P.aux3 + 1, (unsigned long long)nulls);
+}
+
+#define RF_UNION_KERNELS(T)                                                                               \
+    extern "C" __global__ void __launch_bounds__(256) rf_u_part(const __grid_constant__ RfParams P)      \
+    {                                                                                                    \
+        rf_u_part_all(P);                                                                                \
+    }                                                                                                    \
+    extern "C" __global__ void __launch_bounds__(T) rf_u_count(const __grid_constant__ RfParams P)       \
+    {                                                                                                    \
+        rf_u_count_all<T>(P);                                                                            \
+    }                                                                                                    \
+    extern "C" __global__ void __launch_bounds__(T) rf_u_emit(const __grid_constant__ RfParams P)        \
+    {                                                                                                    \
+        rf_u_emit_all<T>(P);                                                                             \
+    }
+#endif  // RF_UNION
 
 // ---------------------------------------------------------------------------------------
 // Template 4: segmented reduce over run-end encoded rows (an Op over a 2-d vector whose output

@@ -2927,22 +2927,24 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             plan_.kernels.push_back({"rf_range", 32, 0, KernelSpec::RANGE});
             plan_.device_range = true;
         }
-        o << "RF_DEV long long rf_lower_bound(const RfCol& c, long long lo, long long hi, " << Ty << " key)\n{\n";
-        o << "    while (lo < hi) { long long mid = (lo + hi) >> 1; if (rf_ld<" << Ty << ">(c.data, mid) < key) lo = mid + 1; else hi = mid; }\n";
-        o << "    return lo;\n}\n\n";
+        // the rows the first vector's rows pair with, complemented where that row does not hold the
+        // key, a tile at a time: (long long*)P.aux5, P.aux_n0 rows to a vector; bounds of the tiles'
+        // windows: (long long*)P.aux4
+        const size_t K = slots.size();
+        auto col0 = [&](size_t k) { return "P.t[" + std::to_string(slots[k]) + "].col[0]"; };
+        o << "#define RF_MERGE 1\n#define RF_MAT_PREP 1\n#define RF_MATERIALIZE 1\n";
+        o << "template <int T>\nRF_DEV void rf_mat_prep(const RfParams& P, long long tile);\n\n";
+        // the match's part of the element functions: the partners' rows, whether all hold the key
         auto body_of = [&](Emitter& E, std::ostringstream& b) -> std::string {
-            std::string a = "P.t[" + std::to_string(slots[0]) + "].col[0]";
-            b << "    const " << Ty << " it = rf_ld<" << Ty << ">(" << a << ".data, r);\n";
-            b << "    const long long rank = r - rf_lower_bound(" << a << ", P.range[0], r, it);\n";
-            b << "    bool mt = rf_valid(" << a << ".valid, r) && it >= (" << Ty << ")P.range[2] && it <= (" << Ty << ")P.range[3];\n";
+            b << "    const " << Ty << " it = rf_ld<" << Ty << ">(" << col0(0) << ".data, r);\n";
+            b << "    bool mt = rf_valid(" << col0(0) << ".valid, r) && it >= (" << Ty << ")P.range[2] && it <= (" << Ty
+              << ")P.range[3];\n";
             E.vec_iter_idx[{sp.vecs[0].second.get(), sp.iter.get()}] = "r";
-            for (size_t k = 1; k < slots.size(); k++) {
-                std::string c = "P.t[" + std::to_string(slots[k]) + "].col[0]";
+            for (size_t k = 1; k < K; k++) {
                 std::string j = "j" + std::to_string(k);
-                b << "    const long long " << j << " = rf_lower_bound(" << c << ", P.range[" << 3 + k << "], " << c
-                  << ".len, it) + rank;\n";
-                b << "    mt = mt && " << j << " < " << c << ".len && rf_ld<" << Ty << ">(" << c << ".data, " << j
-                  << ") == it && rf_valid(" << c << ".valid, " << j << ");\n";
+                b << "    const long long p" << k << " = ((const long long*)P.aux5)[" << k - 1 << " * P.aux_n0 + r], " << j
+                  << " = p" << k << " < 0 ? ~p" << k << " : p" << k << ";\n";
+                b << "    mt = mt && p" << k << " >= 0 && rf_valid(" << col0(k) << ".valid, " << j << ");\n";
                 E.vec_iter_idx[{sp.vecs[k].second.get(), sp.iter.get()}] = j;
             }
             E.bind(op.iters[0], E.scalar("it", sp.iter->type));
@@ -2977,14 +2979,48 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             for (auto& dcl : E.decls) o << "    " << dcl << "\n";
             o << w.str() << "}\n\n";
         }
-        o << "#define RF_MATERIALIZE 1\n#include \"rf_templates.cuh\"\n";
+        o << "#include \"rf_templates.cuh\"\n\n";
+        // per tile boundary: the rank of its first row, then the start of its window in each vector
+        o << "extern \"C\" __global__ void __launch_bounds__(256) rf_merge_part(const __grid_constant__ RfParams P)\n{\n"
+          << "    const long long t = (blockIdx.x * 256ll + threadIdx.x) >> 5, n = " << col0(0) << ".len;\n"
+          << "    if (t > rf_mat_ntiles(P)) return;\n"
+          << "    long long* out = (long long*)P.aux4 + t * " << K << ";\n"
+          << "    const long long x = t * RF_MAT_TILE;\n    long long v[" << K << "];\n"
+          << "    if (x < n) {\n        const " << Ty << " key = rf_key<" << Ty << ">(" << col0(0) << ", x);\n"
+          << "        v[0] = rf_merge_rank<" << Ty << ">(" << col0(0) << ", P.range[0], x, key);\n";
+        for (size_t k = 1; k < K; k++)
+            o << "        v[" << k << "] = rf_merge_bound<" << Ty << ">(" << col0(k) << ", P.range[" << 3 + k << "], key);\n";
+        o << "    } else {\n        v[0] = 0;\n";
+        for (size_t k = 1; k < K; k++) o << "        v[" << k << "] = " << col0(k) << ".len;\n";
+        o << "    }\n    if ((threadIdx.x & 31) == 0)\n        for (int k = 0; k < " << K << "; k++) out[k] = v[k];\n}\n\n";
+        o << "template <int T>\nRF_DEV void rf_mat_prep(const RfParams& P, long long tile)\n{\n"
+          << "    constexpr int R = RF_MAT_TILE / T;\n    __shared__ RfMergeBuf<" << Ty << "> B;\n"
+          << "    const long long* part = (const long long*)P.aux4 + tile * " << K << ";\n"
+          << "    const long long r0 = tile * RF_MAT_TILE, left = P.row_hi - r0;\n"
+          << "    const int n = left < RF_MAT_TILE ? (int)left : RF_MAT_TILE;\n"
+          << "    rf_merge_load<T>(B, " << col0(0) << ", r0, n);\n    long long j[R];\n";
+        for (size_t k = 1; k < K; k++) {
+            o << "    {\n        const RfCol& b = " << col0(k) << ";\n"
+              << "#pragma unroll\n        for (int q = 0; q < R; q++) j[q] = -1;\n"
+              << "        rf_merge_walk<T>(B, r0, n, P.range[0], __ldg(part), b, __ldg(part + " << k << "), __ldg(part + " << K + k
+              << "),\n                         [&](int q, long long, " << Ty << " key, long long lb, long long rank) {\n"
+              << "                             const long long i = lb + rank;\n"
+              << "                             j[q] = i < b.len && rf_key<" << Ty << ">(b, i) == key ? i : ~i;\n                         });\n"
+              // through shared memory, so that whole sectors are written
+              << "#pragma unroll\n        for (int q = 0; q < R; q++) B.win[(int)threadIdx.x * R + q] = j[q];\n        __syncthreads();\n"
+              << "        long long* J = (long long*)P.aux5 + " << k - 1 << " * P.aux_n0 + r0;\n"
+              << "        for (int i = threadIdx.x; i < n; i += T) J[i] = B.win[i];\n        __syncthreads();\n    }\n";
+        }
+        o << "}\n\n";
         o << "RF_MATERIALIZE_KERNELS(" << T << ", " << plan_.out_cols.size() << ")\n";
+        plan_.kernels.push_back({"rf_merge_part", 256, 0, KernelSpec::MERGEPART});
         if (vectorize_) {
             plan_.kernels.push_back({"rf_write_all", T, 0, KernelSpec::FINAL});
         } else {
             plan_.kernels.push_back({"rf_count", T, 0, KernelSpec::COUNT});
             plan_.kernels.push_back({"rf_scatter", T, 0, KernelSpec::SCATTER});
         }
+        plan_.merge_vecs = (int)K;
         plan_.source = o.str();
     }
 
@@ -2995,14 +3031,14 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
     // side's current row (the row holding t, or the lagging side's next row).  Both sides start
     // at row 0 and a side past its end takes no further part (its reads give 0).
     // A key v held cA times in A and cB times in B takes max(cA, cB) visits; visit j of v pairs
-    // A row lA(v) + j with B row lB(v) + j while both exist.  Its position in the walk is
-    //     lA(v) + lB(v) - M(lA(v)) + j,
-    // lX(v) the first row of X with key >= v and M(i) the number of paired A rows before row i.
-    // Kernels: rf_u_flags marks each paired A row, an exclusive scan gives M, rf_u_total the
-    // number of visits, and rf_u_emit lets every A row and every unpaired B row write its visit
-    // at its position - no compaction pass.  iter_cond (a side alive with a valid iterator) is
-    // the validity bit of a vectorised output; without vectorize every visit is a row (inputs
-    // whose iterator columns hold nulls are refused at run time then).
+    // A row lA(v) + j with B row lB(v) + j while both exist (lX the first row of X with key >= v).
+    // So every A row has a visit, at (its row) + U(lB(v)), and every unpaired B row - its rank among
+    // v's rows at or past cA - one at (the A rows up to v) + U(its row), U(i) the number of unpaired B
+    // rows before row i: the kernels of the union section of the templates find those bits and their
+    // prefix counts, the number of visits, and let every row write its visit at its position, with
+    // no compaction pass.  iter_cond (a side alive with a valid iterator) is the validity bit of a
+    // vectorised output; without vectorize every visit is a row (inputs whose iterator columns hold
+    // nulls are refused at run time then).
     void lower_union_op(const Op& op, const Expr& left, const Expr& right)
     {
         plan_.kind = PlanKind::UNION_MERGE;
@@ -3050,23 +3086,10 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
         std::ostringstream o;
         o << "// generated by the reffine_gb300 lowering pass: " << fn_->name << " (union merge co-iteration)\n";
         o << "#include \"rf_device.cuh\"\n\n";
-        o << "// first row of sorted int64 column c (n rows) whose key is >= key (> key when upper)\n";
-        o << "RF_DEV long long rf_u_bound(const RfCol& c, long long n, long long key, bool upper)\n{\n";
-        o << "    long long lo = 0, hi = n;\n    const long long* k = (const long long*)c.data;\n";
-        o << "    while (lo < hi) {\n        const long long m = (lo + hi) >> 1;\n        const long long x = __ldg(k + m);\n";
-        o << "        if (x < key || (upper && x == key)) lo = m + 1; else hi = m;\n    }\n    return lo;\n}\n\n";
-        o << "extern \"C\" __global__ void __launch_bounds__(256) rf_u_flags(const __grid_constant__ RfParams P)\n{\n";
-        o << "    long long* M = (long long*)P.aux4;\n    const long long nA = " << A << ".len, nB = " << B << ".len;\n";
-        o << "    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nA; i += (long long)gridDim.x * blockDim.x) {\n";
-        o << "        const long long v = rf_ld<int64_t>(" << A << ".data, i);\n";
-        o << "        const long long a = i - rf_u_bound(" << A << ", nA, v, false);\n";
-        o << "        const long long lB = rf_u_bound(" << B << ", nB, v, false), cB = rf_u_bound(" << B << ", nB, v, true) - lB;\n";
-        o << "        M[i] = a < cB ? 1 : 0;\n    }\n";
-        o << "    if (blockIdx.x == 0 && threadIdx.x == 0) M[nA] = 0;\n}\n\n";
-        o << "extern \"C\" __global__ void rf_u_total(const __grid_constant__ RfParams P)\n{\n";
-        o << "    if (threadIdx.x != 0 || blockIdx.x != 0) return;\n";
-        o << "    const long long nA = " << A << ".len, nB = " << B << ".len;\n";
-        o << "    ((long long*)P.aux3)[0] = nA + nB - ((const long long*)P.aux4)[nA];\n}\n\n";
+        o << "#define RF_MERGE 1\n#define RF_UNION 1\n#define RF_MATERIALIZE 1\n";
+        o << "RF_DEV const RfCol& rf_u_a(const RfParams& P) { return " << A << "; }\n";
+        o << "RF_DEV const RfCol& rf_u_b(const RfParams& P) { return " << B << "; }\n";
+        if (vectorize_) o << "#define RF_UNION_VALID " << plan_.out_cols.size() << "\n";
         // the visit's outputs
         Emitter E(*this);
         bind_inputs(E);
@@ -3086,37 +3109,10 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
         o << "    const " << ctype(it->type) << " it = (" << ctype(it->type) << ")v;\n";
         for (auto& dcl : E.decls) o << "    " << dcl << "\n";
         o << w.str() << "}\n\n";
-        o << "extern \"C\" __global__ void __launch_bounds__(" << T << ") rf_u_emit(const __grid_constant__ RfParams P)\n{\n";
-        o << "    const long long* M = (const long long*)P.aux4;\n    const long long nA = " << A << ".len, nB = " << B
-          << ".len;\n    const long long V = ((const long long*)P.aux3)[0];\n    long long nulls = 0;\n";
-        o << "    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < nA + nB; r += (long long)gridDim.x * blockDim.x) {\n";
-        o << "        long long v, li, ri, pos;\n";
-        o << "        if (r < nA) {\n            li = r;\n            v = rf_ld<int64_t>(" << A << ".data, li);\n";
-        o << "            const long long lA = rf_u_bound(" << A << ", nA, v, false), a = li - lA;\n";
-        o << "            const long long lB = rf_u_bound(" << B << ", nB, v, false), cB = rf_u_bound(" << B << ", nB, v, true) - lB;\n";
-        o << "            ri = a < cB ? lB + a : lB + cB;\n            pos = lA + lB - M[lA] + a;\n";
-        o << "        } else {\n            ri = r - nA;\n            v = rf_ld<int64_t>(" << B << ".data, ri);\n";
-        o << "            const long long lB = rf_u_bound(" << B << ", nB, v, false), b = ri - lB;\n";
-        o << "            const long long lA = rf_u_bound(" << A << ", nA, v, false), cA = rf_u_bound(" << A << ", nA, v, true) - lA;\n";
-        o << "            if (b < cA) continue;  // paired with A row lA + b, which writes the visit\n";
-        o << "            li = lA + cA;\n            pos = lA + lB - M[lA] + b;\n        }\n";
-        // keys out of order (the walk needs sorted iterator columns) can only move a visit, never
-        // past the output: positions are checked against the visit count
-        o << "        if (pos < 0 || pos >= V) { rf_set_err(P, RF_DEVERR_RANGE); continue; }\n";
-        o << "        rf_u_write(P, li, ri, v, pos);\n";
-        if (vectorize_) {
-            o << "        const bool ok = (li < nA && rf_valid(" << A << ".valid, li)) || (ri < nB && rf_valid(" << B
-              << ".valid, ri));\n";
-            o << "        if (ok)\n            for (int col = 0; col < " << plan_.out_cols.size()
-              << "; col++) atomicOr(P.ov[col] + (pos >> 5), 1u << (pos & 31));\n";
-            o << "        else\n            nulls++;\n";
-        }
-        o << "    }\n";
-        o << "    if (nulls) atomicAdd((unsigned long long*)P.aux3 + 1, (unsigned long long)nulls);\n}\n";
+        o << "#include \"rf_templates.cuh\"\n\nRF_UNION_KERNELS(" << T << ")\n";
         plan_.kernels.clear();
-        plan_.kernels.push_back({"rf_u_flags", 256, 0, KernelSpec::SEGCOUNT});
-        plan_.kernels.push_back({"", 0, 0, KernelSpec::SEGSCAN});
-        plan_.kernels.push_back({"rf_u_total", 32, 0, KernelSpec::RANGE});
+        plan_.kernels.push_back({"rf_u_part", 256, 0, KernelSpec::MERGEPART});
+        plan_.kernels.push_back({"rf_u_count", T, 0, KernelSpec::COUNT});
         plan_.kernels.push_back({"rf_u_emit", T, 0, KernelSpec::SCATTER});
         plan_.source = o.str();
     }

@@ -54,7 +54,7 @@ struct KernelSpec {
     std::string name;
     int threads = 256;
     size_t smem = 0;
-    enum Role { MAIN, RANGE, STOP, COUNT, SCATTER, INIT, FINAL, SEGCOUNT, SEGSCAN, SEGPART, SEGREDUCE, SEGFIX, IXCOUNT,
+    enum Role { MAIN, RANGE, STOP, COUNT, SCATTER, INIT, FINAL, SEGPART, SEGREDUCE, SEGFIX, MERGEPART, IXCOUNT,
                 IXINIT, IXBUILD } role = MAIN;
 };
 
@@ -85,6 +85,7 @@ struct Plan {
     size_t acc_bytes = 0;               // bytes of one unit's partial (scan-reduce, segmented reduce)
     int seg_items = 0;                  // segmented reduce: rows and run ends of a tile
     int ixf_input = -1;                 // input whose index a run replaces by a filtered one (-1: none)
+    int merge_vecs = 0;                 // merge join: vectors walked together
     int union_inputs[2] = {-1, -1};     // union merge: the two merged vectors (Func inputs)
     int hg_hot = 0;                     // hash group-by: hottest keys folded per warp (index 2x)
     int hg_warm = 0;                    // hash group-by: further hot keys in shared memory (index 2x)

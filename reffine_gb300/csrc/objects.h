@@ -202,7 +202,7 @@ struct rf_plan {
     unsigned long long ixf_buf_for = 0;
     RfIndex ixf_ix{};
     cudaEvent_t ixf_ev = nullptr;     // recorded after the last run that read ixf_buf
-    // segmented reduce
+    // segmented reduce: tile bounds, states; merges: tile bounds, partner rows
     long long* seg_woff = nullptr;
     long long* seg_tmp = nullptr;
     void* seg_part = nullptr;

@@ -2214,10 +2214,10 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     P.aux1 = p->d_tiles;
     P.aux2 = (unsigned char*)p->d_tiles + bit_bytes;
     P.aux3 = p->d_res;
-    long long nruns = 0, seg_tiles = 0;
+    long long seg_tiles = 0;
     if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
         rf_table* vt = args[pl.drive_input].table;
-        nruns = vt->cols[0].nvals;
+        const long long nruns = vt->cols[0].nvals;
         const long long nrows = vt->cols[0].logical;
         seg_tiles = (nruns + nrows + pl.seg_items - 1) / pl.seg_items;
         if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(seg_tiles + 1) * 8, s) ||
@@ -2230,6 +2230,18 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         P.aux_n0 = nrows;
         P.aux_n1 = seg_tiles;
     }
+    if (pl.kind == rfg::PlanKind::MERGE_JOIN) {
+        // [tiles + 1][vectors] bounds; a partner row for each row of the first vector in each other one
+        const long long n = std::max<long long>(hi - lo, 1);
+        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(ntiles + 1) * pl.merge_vecs * 8, s) ||
+            !grow(&p->seg_part, &p->seg_part_cap, (size_t)n * (pl.merge_vecs - 1) * 8, s)) {
+            free_table_mem(t.get());
+            return fail(ctx, RF_ERR_OOM, "merge buffers");
+        }
+        P.aux4 = p->seg_woff;
+        P.aux5 = p->seg_part;
+        P.aux_n0 = n;
+    }
     if (union_merge) {
         // paired-row counts of the first vector, scanned in place (nA + 1 entries)
         rf_table* ta = args[pl.union_inputs[0]].table;
@@ -2239,13 +2251,20 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
             return fail(ctx, RF_ERR_UNSUPPORTED,
                         "a union over iterator columns with nulls is lowered in the vectorised form only");
         }
-        nruns = ta->cols[0].nvals + 1;
-        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(nruns + 1) * 8, s) ||
-            !grow((void**)&p->seg_tmp, &p->seg_tmp_cap, (size_t)(nruns / 2048 + 4) * 8, s)) {
+        // tiles of each side, the bounds of both, a word of prefix counts per 64 rows of the second
+        // side and the rows its unpaired ones follow
+        const long long nb = tb->cols[0].nvals;
+        P.aux_n0 = (ta->cols[0].nvals + RF_MAT_TILE - 1) / RF_MAT_TILE;
+        P.aux_n1 = (nb + RF_MAT_TILE - 1) / RF_MAT_TILE;
+        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(P.aux_n0 + P.aux_n1 + 2) * 16, s) ||
+            !grow((void**)&p->seg_tmp, &p->seg_tmp_cap, (size_t)(P.aux_n1 + 1) * (RF_MAT_TILE / 16), s) ||
+            !grow(&p->seg_part, &p->seg_part_cap, (size_t)(nb + 1) * 8, s)) {
             free_table_mem(t.get());
             return fail(ctx, RF_ERR_OOM, "union merge buffers");
         }
         P.aux4 = p->seg_woff;
+        P.aux0 = p->seg_tmp;
+        P.aux5 = p->seg_part;
     }
     int units = units_for(p, ntiles);
     P.nunits = units;
@@ -2274,20 +2293,13 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
             }
             cap = total;
         }
-        if (k.role == rfg::KernelSpec::SEGSCAN) {
-            int e = rf_k_scan_excl(p->seg_woff, nruns, p->seg_tmp, s);
-            if (e) {
-                free_table_mem(t.get());
-                return fail(ctx, RF_ERR_CUDA, "segment scan launch: %s", cudaGetErrorString((cudaError_t)e));
-            }
-            ctx->launches += 3;
-            continue;
-        }
         int grid = units;
-        if (k.role == rfg::KernelSpec::SEGCOUNT || k.role == rfg::KernelSpec::INIT) grid = ctx->sm_count * 8;
+        if (k.role == rfg::KernelSpec::INIT) grid = ctx->sm_count * 8;
         if (k.role == rfg::KernelSpec::SEGPART) grid = (int)(seg_tiles / 8 + 1);  // a warp per tile boundary
         if (k.role == rfg::KernelSpec::SEGREDUCE) grid = (int)std::max<long long>(seg_tiles, 1);
         if (k.role == rfg::KernelSpec::SEGFIX) grid = 1;
+        if (k.role == rfg::KernelSpec::MERGEPART)
+            grid = (int)((union_merge ? P.aux_n0 + P.aux_n1 + 1 : ntiles) / 8 + 1);
         if (pl.kind == rfg::PlanKind::HASH_GROUP && k.role == rfg::KernelSpec::MAIN)
             grid = std::max(1, p->max_units * t_grid_share / 100);
         // the materialisation kernels take a tile a block, as many blocks as fill the GPU four times

@@ -45,3 +45,47 @@ def test_compaction_at_tile_edges(eng, vectorize, n, after):
         np.testing.assert_array_equal(got, v)
         for g, r in zip(out["cols"], ref["cols"]):
             np.testing.assert_array_equal(g[v], r[v])
+
+
+def key_table(keys, seed=0):
+    keys = np.asarray(keys, dtype=np.int64)
+    v = np.random.default_rng(seed + len(keys)).integers(-1000, 1000, len(keys))
+    return Table.from_arrays(1, {"k": keys, "v": v})
+
+
+def spread(n, hi, seed):
+    k = np.sort(np.random.default_rng(seed).integers(0, hi, n))
+    k[0] = 0
+    return k
+
+
+MERGES = {  # left, right: long runs of one key across tiles, windows larger than the buffer, sides that end first
+    "equal_runs": ([0] + [7] * 5000 + [9] * 3, [0] + [7] * 4500 + [8] * 2100 + [9]),
+    "sparse_left": ([0, 40_000, 40_001, 99_999], spread(60_000, 100_000, 1)),
+    "sparse_right": (spread(60_000, 100_000, 2), [0, 1, 50_000, 99_999, 99_999]),
+    "tile": (np.arange(2048), np.arange(0, 4096, 2)), "tile_plus": (np.arange(2049) // 2, np.arange(4097) // 3),
+    "ends_first": (spread(5000, 1000, 3), spread(5000, 30_000, 4)), "one": ([0], [0]),
+    "clusters": (np.repeat(np.arange(0, 60_000, 3000), 700), np.concatenate([[0], np.arange(1, 50_000), [57_000] * 5000])),
+}
+
+
+@pytest.mark.parametrize("vectorize", [False, True])
+@pytest.mark.parametrize("mode", ["inner", "outer"])
+@pytest.mark.parametrize("name", list(MERGES))
+def test_merges_at_tile_edges(eng, name, mode, vectorize):
+    a, b = (key_table(k, i) for i, k in enumerate(MERGES[name]))
+    t, left, right = _sym("t", _i64_t), _sym("left", a.get_data_type()), _sym("right", b.get_data_type())
+    space = _in(t, left) & _in(t, right) if mode == "inner" else _in(t, left) | _in(t, right)
+    op = _op([t], space, [_get(left[t], 0), _get(right[t], 0)])
+    os_ = _sym("op", op)
+    fn = _func("merge", os_, [left, right])
+    fn.tbl[os_] = op
+    out = plan_run_table(eng, eng.compile(fn, vectorize), a, b)
+    ref = loopgen.Query(fn, vectorize)(a, b)
+    if mode == "inner" and vectorize:  # the plan emits the left side's rows, null where they pair with none
+        v = np.ones(out["len"], bool) if out["valid"][0] is None else out["valid"][0]
+        w = np.ones(ref["len"], bool) if ref["valid"] is None else ref["valid"]
+        for g, r in zip(out["cols"], ref["cols"]):
+            np.testing.assert_array_equal(g[v], r[w])
+    else:
+        assert_table_same(out, ref)
