@@ -69,6 +69,8 @@ typedef struct RfParams {
     int flags;
     int unit0;                 // first unit of this launch (a launch runs units unit0 .. unit0+grid-1)
     int rsv_;
+    long long* host_rows;      // table outputs: where a count of rows is left for the host (pinned)
+    long long out_rows;        // table outputs: rows, once counted
     void* oc[RF_MAX_COLS];     // table outputs: column values
     unsigned* ov[RF_MAX_COLS]; // table outputs: validity words (vectorised)
 } RfParams;

@@ -350,8 +350,9 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
 // tile's keys begin (they end where the next tile's begin), and rf_merge_walk copies the tile's keys
 // and that window into shared memory, where a thread searches once for its first row and walks on
 // for the others.  A window larger than the buffer is searched in place.  The keys are so read
-// once; the walk's shared-memory latency is covered by the other blocks of the SM.  (Two binary
-// searches of the whole columns a row, in each of two kernels: 3.8 ms for 5M rows against 4M.)
+// once; the walk's shared-memory latency is covered by the other blocks of the SM.  (5M rows
+// against 4M: 3836 us a call with two binary searches of the whole columns a row in each of two
+// kernels on one block an SM, 580 us with the GPU full of them, 191 us so.)
 // Keys out of order give other partners, never an access outside the columns.
 // ---------------------------------------------------------------------------------------
 #ifdef RF_MERGE
@@ -461,7 +462,7 @@ RF_DEV void rf_merge_walk(RfMergeBuf<K>& B, long long r0, int n, long long from,
 //   and with RF_MAT_PREP rf_mat_prep<T>(P, tile), which a block runs before the tile's conditions.
 //   Output columns: P.oc[c]; validity words: P.ov[c]; a bit per element that passes, 32 elements
 //   from P.row_lo on to a word: (unsigned*)P.aux1; per-tile counts / offsets: (long long*)P.aux2;
-//   results (long long*)P.aux3: [0] = rows written, [1] = null count.
+//   the number that pass goes to *P.host_rows, the null count to *(long long*)P.aux3.
 //   Compaction (vectorize off) keeps passing elements in loop order: rf_count evaluates the
 //   condition once, writes its bits and each tile's count, and its last block turns the counts
 //   into offsets; rf_scatter lists a tile's passing elements in shared memory and emits them 256
@@ -504,9 +505,9 @@ RF_DEV int rf_block_sum_int(int v, int* sh)
     return t;
 }
 
-// exclusive scan of n tile counts in place by one block; total -> *total
+// exclusive scan of n tile counts in place by one block; returns the total
 template <int T>
-RF_DEV void rf_mat_scan(long long* cnt, long long n, long long* total)
+RF_DEV long long rf_mat_scan(long long* cnt, long long n)
 {
     constexpr int K = 8;  // counts a thread scans in its registers per step
     __shared__ long long wsum[T / 32];
@@ -542,7 +543,7 @@ RF_DEV void rf_mat_scan(long long* cnt, long long n, long long* total)
         carry += all;
         __syncthreads();  // wsum is rewritten by the next step
     }
-    if (threadIdx.x == 0) *total = carry;
+    return carry;
 }
 
 #ifndef RF_UNION  // (a union writes its visits itself)
@@ -582,8 +583,11 @@ RF_DEV void rf_mat_count(const RfParams& P)
     __syncthreads();
     if (!last) return;
     __threadfence();
-    rf_mat_scan<T>(cnt, nt, (long long*)P.aux3);
-    if (threadIdx.x == 0) *P.counter = 0u;
+    const long long total = rf_mat_scan<T>(cnt, nt);
+    if (threadIdx.x == 0) {
+        *P.host_rows = total;
+        *P.counter = 0u;
+    }
 }
 
 template <int T>
@@ -662,7 +666,7 @@ RF_DEV void rf_mat_write_all(const RfParams& P, int ncols)
             }
         }
     }
-    if (lane == 0 && nulls) atomicAdd((unsigned long long*)P.aux3 + 1, (unsigned long long)nulls);
+    if (lane == 0 && nulls) atomicAdd((unsigned long long*)P.aux3, (unsigned long long)nulls);
 }
 
 #define RF_MATERIALIZE_KERNELS(T, NCOLS)                                                                  \
@@ -688,10 +692,11 @@ RF_DEV void rf_mat_write_all(const RfParams& P, int ncols)
 //   (long long*)P.aux4: {rank, window start} of each tile boundary of A (P.aux_n0 tiles + 1), then of
 //   B (P.aux_n1 + 1); (long long*)P.aux5: of each B row, the A rows up to its key if it is unpaired,
 //   else -1; (unsigned*)P.aux1: a bit per B row, unpaired; (unsigned short*)P.aux0: unpaired rows of
-//   the tile before each word; (long long*)P.aux2: and of the tiles before each tile; P.aux3[0]: visits.
+//   the tile before each word; (long long*)P.aux2: and of the tiles before each tile; visits: *P.host_rows, then P.out_rows.
 // Both key columns are read twice (once to find what is unpaired, once to write); the rest of the
-// traffic is the outputs.  (3M rows against 2.5M with 40 % of the keys shared: 1728 us a call with
-// three binary searches a row in each of two kernels on one block an SM.)
+// traffic is the outputs.  (3M rows against 2.5M with 40 % of the keys shared: 1749 us a call with
+// three binary searches a row in each of two kernels on one block an SM, 657 us with the GPU full of
+// them, 282 us so.)
 // ---------------------------------------------------------------------------------------
 #ifdef RF_UNION
 // the first row of c at or after lo with a key above `key`, knowing that row hi has one (or is the end)
@@ -790,9 +795,9 @@ RF_DEV void rf_u_count_all(const RfParams& P)
     __syncthreads();
     if (!last) return;
     __threadfence();
-    rf_mat_scan<T>(cnt, P.aux_n1, (long long*)P.aux3);
+    const long long total = rf_mat_scan<T>(cnt, P.aux_n1);
     if (threadIdx.x == 0) {
-        ((long long*)P.aux3)[0] += a.len;
+        *P.host_rows = a.len + total;
         *P.counter = 0u;
     }
 }
@@ -824,7 +829,7 @@ RF_DEV void rf_u_emit_all(const RfParams& P)
     const long long* off = (const long long*)P.aux2;
     const unsigned* bits = (const unsigned*)P.aux1;
     const unsigned short* before = (const unsigned short*)P.aux0;
-    const long long V = ((const long long*)P.aux3)[0];
+    const long long V = P.out_rows;
     long long nulls = 0;
     for (long long tile = blockIdx.x; tile < P.aux_n0 + P.aux_n1; tile += gridDim.x) {
         if (tile < P.aux_n0) {  // a tile of A: every row has a visit
@@ -873,7 +878,7 @@ RF_DEV void rf_u_emit_all(const RfParams& P)
         }
         __syncthreads();
     }
-    if (nulls) atomicAdd((unsigned long long*)P.aux3 + 1, (unsigned long long)nulls);
+    if (nulls) atomicAdd((unsigned long long*)P.aux3, (unsigned long long)nulls);
 }
 
 #define RF_UNION_KERNELS(T)                                                                               \
@@ -907,7 +912,7 @@ RF_DEV void rf_u_emit_all(const RfParams& P)
 // row order, by the tiles alone, so the bits do not depend on the scheduling.  Bound by reading
 // the rows: they are staged through shared memory, whole sectors a warp, and so are the run ends.
 // (20M rows of one double in 2M Zipf(1.1) runs: 2.37 ms a call with a thread to each 256 rows of a
-// run and one thread folding a run's pieces in turn, of which 1.94 ms were those folds; 0.33 ms so.)
+// run and one thread folding a run's pieces in turn, of which 1.94 ms were those folds; 0.23 ms so.)
 // ---------------------------------------------------------------------------------------
 #ifdef RF_SEG_REDUCE
 RF_DEV long long rf_seg_end(const RfParams& P, long long run)

@@ -92,7 +92,7 @@ struct rf_ctx {
     std::atomic<long long> launches{0};
     int sm_count = 0;
     int pageable_direct = 0;  // cudaDevAttrPageableMemoryAccessUsesHostPageTables
-    int* dev_err = nullptr;  // device error word shared by this context's launches
+    int* dev_err = nullptr;  // error word shared by this context's launches (pinned host memory)
     // autotuner choices: tile rows per (query shape key, log2 row-count bucket)
     std::mutex tune_mu;
     std::map<std::string, std::map<int, long long>> tune;
@@ -173,7 +173,7 @@ struct rf_plan {
     int reduce_units = 0;             // work units a reduce may be cut into (units_for)
     int thunk_slot = -1;
     long long tile_override = 0;      // set while the autotuner times a candidate
-    unsigned char* h_res = nullptr;   // pinned: [error word, 16 B][value result]
+    unsigned char* h_res = nullptr;   // pinned: the value result, or [rows, nulls, loop range] of a table
     // batched execution (value-output plans without device-computed loop bounds)
     CUfunction batch_fn = nullptr;
     int batch_grid = 0;
@@ -182,7 +182,7 @@ struct rf_plan {
     // table outputs
     long long* d_tiles = nullptr;     // a bit per element, then per-tile counts / offsets
     size_t tiles_cap = 0;             // bytes
-    long long* d_res = nullptr;       // [rows written, null count]
+    long long* d_res = nullptr;       // null count
     // hash group-by
     void* hg_keys = nullptr;
     void* hg_acc = nullptr;

@@ -371,8 +371,10 @@ extern "C" int rf_gpu_init(int device, rf_ctx** out)
         const char* mb = getenv("RF_IXF_CACHE_MB");
         ctx->ixf_budget = (size_t)(mb ? atoll(mb) : 2048) << 20;
     }
-    CUDA_TRY(nullptr, cudaMalloc((void**)&ctx->dev_err, sizeof(int)));
-    CUDA_TRY(nullptr, cudaMemset(ctx->dev_err, 0, sizeof(int)));
+    // the error word is pinned host memory that kernels write in place: only a failing run touches it,
+    // and the host reads it after a synchronisation without a copy
+    CUDA_TRY(nullptr, cudaHostAlloc((void**)&ctx->dev_err, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    *ctx->dev_err = 0;
     // rf_plan_run_noalloc's fixed array: with lazy module loading the array's device memory is
     // set up when its module first loads, so the address is looked up here (loading the module
     // while the caller may still allocate), never inside a run that promises no allocation
@@ -381,7 +383,7 @@ extern "C" int rf_gpu_init(int device, rf_ctx** out)
         size_t scratch_bytes = 0;
         int e = rf_k_noalloc_scratch(device, &scratch, &scratch_bytes);
         if (e) {
-            cudaFree(ctx->dev_err);
+            cudaFreeHost(ctx->dev_err);
             cudaStreamDestroy(ctx->stream);
             return RF_ERR_CUDA;
         }
@@ -396,7 +398,7 @@ extern "C" int rf_gpu_shutdown(rf_ctx* ctx)
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     ctx->modules.clear();
-    cudaFree(ctx->dev_err);
+    cudaFreeHost(ctx->dev_err);
     if (ctx->stage) cudaFreeHost(ctx->stage);
     for (auto& e : ctx->pipe_ev) cudaEventDestroy(e);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
@@ -425,17 +427,12 @@ extern "C" int rf_ctx_stream(rf_ctx* ctx, void** stream)
 }
 
 namespace rfrt {
-int check_device_error(rf_ctx* ctx)
-{
-    int e = 0;
-    CUDA_TRY(ctx, cudaMemcpy(&e, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost));
-    return device_error(ctx, e);
-}
+int check_device_error(rf_ctx* ctx) { return device_error(ctx, *(volatile int*)ctx->dev_err); }
 
 int device_error(rf_ctx* ctx, int e)
 {
     if (e) {
-        cudaMemset(ctx->dev_err, 0, sizeof(int));
+        *(volatile int*)ctx->dev_err = 0;
         const char* what = e == RF_DEVERR_PROBE ? "hash probe exhausted the table"
                            : e == RF_DEVERR_WAIT ? "bounded wait ran out"
                            : e == RF_DEVERR_RANGE ? "loop lower bound not found in the iterator column (Locate returned -1)"
@@ -1091,7 +1088,7 @@ int build_plan(rf_ctx* ctx, const std::shared_ptr<reffine::Func>& fn, bool vecto
     // the plan's own device buffers, carved from one allocation of the context's stream-ordered
     // pool (compiling many plans costs no device-wide synchronisation):
     //   [partials of the units][completion counter 64 B][loop range 64 B][value result]
-    //   [table outputs: results 64 B]
+    //   [table outputs: null count 64 B]
     p->partials_bytes = (size_t)p->reduce_units * (p->plan.acc_bytes ? p->plan.acc_bytes : 8);
     const size_t osz = p->plan.out_size ? p->plan.out_size : 8;
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
@@ -1346,7 +1343,7 @@ int fill_params(rf_plan* p, const rf_arg* args, int n_args, RfParams& P, long lo
     P.range = pl.device_range ? p->range : nullptr;
     P.partials = p->partials;
     P.counter = p->counter;
-    P.out = p->dout;
+    P.out = p->dout;  // (runs that hand the result to the host or to the caller's buffer set their own)
     P.err = ctx->dev_err;
     return RF_OK;
 }
@@ -1464,7 +1461,7 @@ void release_filtered_index(rf_plan* p, cudaStream_t s)
     p->ixf_buf_for = 0;
 }
 
-int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, RfParams* Pout)
+int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, void* out)
 {
     rf_ctx* ctx = p->ctx;
     RfParams P;
@@ -1475,6 +1472,7 @@ int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, RfParams
     long long ntiles = (hi - lo + P.tile_rows - 1) / P.tile_rows;
     int units = units_for(p, ntiles);
     P.nunits = units;
+    if (out) P.out = (unsigned char*)out;
     void* ixbuf = nullptr;
     std::unique_lock<std::mutex> ixf_lock(ctx->ixf_mu, std::defer_lock);
     if (pl.ixf_input >= 0) {
@@ -1500,8 +1498,17 @@ int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, RfParams
     if (ixbuf) cudaFreeAsync(ixbuf, s);  // after the kernels that read it, in stream order
     if (p->ixf_buf && ixf_lock.owns_lock()) cudaEventRecord(p->ixf_ev, s);  // the kept index's last use
     if (ixf_lock.owns_lock()) ixf_lock.unlock();
-    if (rc) return rc;
-    if (Pout) *Pout = P;
+    return rc;
+}
+
+// pinned host memory for what a run hands back: a value result (written there by the kernel that
+// finishes it), or the counts of a table result
+int result_buffer(rf_plan* p)
+{
+    if (p->h_res) return RF_OK;
+    const size_t bytes = std::max<size_t>(p->plan.out_is_table ? 0 : p->plan.out_size, 64);
+    if (cudaHostAlloc((void**)&p->h_res, bytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+        return fail(p->ctx, RF_ERR_OOM, "pinned result buffer");
     return RF_OK;
 }
 
@@ -1556,12 +1563,12 @@ int run_streamed(rf_plan* p, const rf_arg* args, int n_args, const std::vector<H
             CUDA_TRY(ctx, cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyHostToDevice, s));
         return rf_plan_run(p, args, n_args, out, s);
     }
-    if (!p->h_res && cudaHostAlloc((void**)&p->h_res, 16 + p->plan.out_size, cudaHostAllocDefault) != cudaSuccess)
-        return fail(ctx, RF_ERR_OOM, "pinned result buffer");
     RfParams P;
     long long lo, hi;
-    int rc = fill_params(p, args, n_args, P, lo, hi, true);
+    int rc = result_buffer(p);
+    if (!rc) rc = fill_params(p, args, n_args, P, lo, hi, true);
     if (rc) return rc;
+    P.out = p->h_res;
     const rfg::Plan& pl = p->plan;
     const long long tr = P.tile_rows;
     const long long ntiles = (hi - lo + tr - 1) / tr;
@@ -1637,13 +1644,9 @@ int run_streamed(rf_plan* p, const rf_arg* args, int n_args, const std::vector<H
         cudaStreamSynchronize(s);
         return rc;
     }
-    CUDA_TRY(ctx, cudaMemcpyAsync(p->h_res, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(ctx, cudaMemcpyAsync(p->h_res + 16, p->dout, pl.out_size, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(ctx, cudaStreamSynchronize(s));  // after the last chunk's event: every copy has landed too
-    int e;
-    memcpy(&e, p->h_res, sizeof(int));
-    if ((rc = device_error(ctx, e))) return rc;
-    if (out) memcpy(out, p->h_res + 16, pl.out_size);
+    if ((rc = check_device_error(ctx))) return rc;
+    if (out) memcpy(out, p->h_res, pl.out_size);
     return RF_OK;
 }
 
@@ -1934,9 +1937,18 @@ extern "C" int rf_plan_launch(rf_plan* p, const rf_arg* args, int32_t n_args, vo
     cudaSetDevice(ctx->device);
     if (p->plan.out_is_table) return fail(ctx, RF_ERR_INVALID, "rf_plan_launch takes value-output plans");
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    int rc = enqueue(p, args, n_args, s, nullptr);
+    // the kernel that finishes the result writes it to the caller's buffer where that is aligned for
+    // its fields (and is device memory, or pinned host memory: a copy takes any other)
+    bool direct = dev_out && ((uintptr_t)dev_out & 15) == 0;
+    if (direct) {
+        cudaPointerAttributes a;
+        direct = cudaPointerGetAttributes(&a, dev_out) == cudaSuccess && a.type == cudaMemoryTypeDevice && a.device == ctx->device;
+        cudaGetLastError();
+    }
+    int rc = enqueue(p, args, n_args, s, direct ? dev_out : nullptr);
     if (rc) return rc;
-    if (dev_out) CUDA_TRY(ctx, cudaMemcpyAsync(dev_out, p->dout, p->plan.out_size, cudaMemcpyDeviceToDevice, s));
+    if (dev_out && !direct)
+        CUDA_TRY(ctx, cudaMemcpyAsync(dev_out, p->dout, p->plan.out_size, cudaMemcpyDeviceToDevice, s));
     return RF_OK;
 }
 
@@ -2210,10 +2222,19 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         free_table_mem(t.get());
         return fail(ctx, RF_ERR_OOM, "tile buffer allocation failed");
     }
-    CUDA_TRY(ctx, cudaMemsetAsync(p->d_res, 0, 64, s));
+    // rows written and nulls: a compaction's last block leaves its count in pinned host memory; the
+    // null rows of a vectorised one are counted with atomics, on the device
+    if ((rc = result_buffer(p))) {
+        free_table_mem(t.get());
+        return rc;
+    }
+    volatile long long* h_counts = (volatile long long*)p->h_res;
+    for (int i = 0; i < 4; i++) h_counts[i] = 0;
+    if (pl.vectorize) CUDA_TRY(ctx, cudaMemsetAsync(p->d_res, 0, 64, s));
     P.aux1 = p->d_tiles;
     P.aux2 = (unsigned char*)p->d_tiles + bit_bytes;
     P.aux3 = p->d_res;
+    P.host_rows = (long long*)p->h_res;
     long long seg_tiles = 0;
     if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
         rf_table* vt = args[pl.drive_input].table;
@@ -2271,9 +2292,8 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     for (size_t i = 0; i < pl.kernels.size(); i++) {
         const auto& k = pl.kernels[i];
         if ((int)i == iscatter) {
-            long long total = 0;
-            CUDA_TRY(ctx, cudaMemcpyAsync(&total, p->d_res, 8, cudaMemcpyDeviceToHost, s));
             CUDA_TRY(ctx, cudaStreamSynchronize(s));
+            const long long total = h_counts[0];
             if ((rc = check_device_error(ctx))) {
                 free_table_mem(t.get());
                 if (pl.kind == rfg::PlanKind::HASH_GROUP && rc == RF_ERR_DEVICE && hg_cap < (1LL << 34) &&
@@ -2292,6 +2312,7 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
                 return rc;
             }
             cap = total;
+            P.out_rows = total;
         }
         int grid = units;
         if (k.role == rfg::KernelSpec::INIT) grid = ctx->sm_count * 8;
@@ -2313,9 +2334,9 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
             return rc;
         }
     }
-    long long res[2] = {0, 0}, rng[2] = {lo, hi};
-    CUDA_TRY(ctx, cudaMemcpyAsync(res, p->d_res, 16, cudaMemcpyDeviceToHost, s));
-    if (pl.device_range) CUDA_TRY(ctx, cudaMemcpyAsync(rng, p->range, 16, cudaMemcpyDeviceToHost, s));
+    const bool visits = pl.vectorize && !union_merge;  // every visited element is a row
+    if (pl.vectorize) CUDA_TRY(ctx, cudaMemcpyAsync(p->h_res + 8, p->d_res, 8, cudaMemcpyDeviceToHost, s));
+    if (visits && pl.device_range) CUDA_TRY(ctx, cudaMemcpyAsync(p->h_res + 16, p->range, 16, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(ctx, cudaStreamSynchronize(s));
     rc = check_device_error(ctx);
     if (rc) {
@@ -2327,16 +2348,17 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         }
         return rc;
     }
-    long long rows = res[0];
-    if (pl.vectorize && !union_merge) {
-        long long a = std::max(lo, rng[0]), b = std::min(hi, rng[1]);
+    long long rows = h_counts[0];
+    if (visits) {
+        const long long a = pl.device_range ? std::max<long long>(lo, (long long)h_counts[2]) : lo;
+        const long long b = pl.device_range ? std::min<long long>(hi, (long long)h_counts[3]) : hi;
         rows = b > a ? b - a : 0;
     }
     if (rows > cap) {
         free_table_mem(t.get());
         return fail(ctx, RF_ERR_DEVICE, "materialisation wrote %lld rows into %lld", rows, cap);
     }
-    t->null_count = pl.vectorize ? res[1] : 0;
+    t->null_count = pl.vectorize ? h_counts[1] : 0;
     for (auto& dc : t->cols) {
         dc.nvals = rows;
         dc.logical = rows;
@@ -2374,9 +2396,9 @@ extern "C" int rf_plan_run_noalloc(rf_plan* p, const rf_arg* args, int32_t n_arg
     if (rc) return rc;
     long long ntiles = (hi - lo + P.tile_rows - 1) / P.tile_rows;
     int units = units_for(p, ntiles);
-    // layout: [counter 256][loop bounds 256][error word at 752][result at 768, 256-aligned]
+    // layout: [counter 256][loop bounds 256][unused][result at 768, 256-aligned]
     // [partials: units x max(acc_bytes, 8); every unit writes at least one 8-byte accumulator]
-    const size_t err_at = 752, out_at = 768;
+    const size_t out_at = 768;
     size_t out_bytes = (pl.out_size + 255) / 256 * 256;
     size_t acc = pl.acc_bytes ? pl.acc_bytes : 8;
     size_t need = out_at + out_bytes + (size_t)units * acc;
@@ -2401,20 +2423,15 @@ extern "C" int rf_plan_run_noalloc(rf_plan* p, const rf_arg* args, int32_t n_arg
                        : units;
         if ((rc = launch(ctx, p->fns[i], grid, k.threads, k.smem, s, &P))) return rc;
     }
-    // the error word is placed just before the result, so one copy brings back both; the result
-    // reaches host_out only once the error word says the run succeeded (as in rf_plan_run)
-    CUDA_TRY(ctx, cudaMemcpyAsync(b + err_at, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToDevice, s));
-    unsigned char small[16 + 4096];
-    const bool one_copy = pl.out_size <= sizeof(small) - 16;
-    const size_t back = one_copy ? 16 + pl.out_size : 16;
-    CUDA_TRY(ctx, cudaMemcpyAsync(small, b + err_at, back, cudaMemcpyDeviceToHost, s));
+    // the result reaches host_out only once the error word says the run succeeded (as in rf_plan_run)
+    unsigned char small[4096];
+    const bool one_copy = pl.out_size <= sizeof(small);
+    if (one_copy) CUDA_TRY(ctx, cudaMemcpyAsync(small, P.out, pl.out_size, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    int err;
-    memcpy(&err, small, sizeof(int));
-    if ((rc = device_error(ctx, err))) return rc;
+    if ((rc = check_device_error(ctx))) return rc;
     if (one_copy) {
-        memcpy(host_out, small + 16, pl.out_size);
-    } else {  // a result larger than the stack buffer: a second copy, after the check
+        memcpy(host_out, small, pl.out_size);
+    } else {  // a result larger than the stack buffer: copied after the check
         CUDA_TRY(ctx, cudaMemcpyAsync(host_out, P.out, pl.out_size, cudaMemcpyDeviceToHost, s));
         CUDA_TRY(ctx, cudaStreamSynchronize(s));
     }
@@ -2432,19 +2449,11 @@ extern "C" int rf_plan_run(rf_plan* p, const rf_arg* args, int32_t n_args, void*
         *(rf_table**)out = nullptr;
         return run_table(p, args, n_args, (rf_table**)out, s);
     }
-    if (!p->h_res) {
-        if (cudaHostAlloc((void**)&p->h_res, 16 + p->plan.out_size, cudaHostAllocDefault) != cudaSuccess)
-            return fail(ctx, RF_ERR_OOM, "pinned result buffer");
-    }
-    int rc = enqueue(p, args, n_args, s, nullptr);
+    int rc = result_buffer(p);
+    if (!rc) rc = enqueue(p, args, n_args, s, p->h_res);
     if (rc) return rc;
-    // the error word and the result come back in one round trip
-    CUDA_TRY(ctx, cudaMemcpyAsync(p->h_res, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(ctx, cudaMemcpyAsync(p->h_res + 16, p->dout, p->plan.out_size, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    int e;
-    memcpy(&e, p->h_res, sizeof(int));
-    if ((rc = device_error(ctx, e))) return rc;
-    if (out) memcpy(out, p->h_res + 16, p->plan.out_size);
+    if ((rc = check_device_error(ctx))) return rc;
+    if (out) memcpy(out, p->h_res, p->plan.out_size);
     return RF_OK;
 }

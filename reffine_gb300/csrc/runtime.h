@@ -11,8 +11,9 @@
 
 namespace rfrt {
 
-// enqueues the kernels of one plan run on stream `s` (no synchronisation)
-int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, RfParams* P);
+// enqueues the kernels of one plan run on stream `s` (no synchronisation); the value result goes to
+// `out` (device memory, or pinned host memory), NULL: to the plan's own device buffer
+int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, void* out);
 // fills the parameter block of a plan run; lo/hi = tiling range
 int fill_params(rf_plan* p, const rf_arg* args, int n_args, RfParams& P, long long& lo, long long& hi,
                 bool may_allocate);
