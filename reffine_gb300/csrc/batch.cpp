@@ -4,8 +4,8 @@
 // The reference runs one query per call (compile_op's function, include/reffine/utils/utils.h:
 // 47-54) and has no batching; this is the GB300 side's serving primitive.  A batch holds Reduce
 // queries of any shapes.  Queries sharing a compiled shape run in one launch of that shape's
-// rf_batch kernel (device/rf_templates.cuh), a persistent kernel whose blocks walk a work list
-// of (query, unit) items; every query is cut into the units of its stand-alone launch and folded
+// rf_batch kernel (device/rf_templates.cuh), a persistent kernel whose blocks walk the units of
+// all its queries; every query is cut into the units of its stand-alone launch and folded
 // in the same order, so each result has the same bits alone or in the mix.  The launch sequence
 // (parameter and work-list copies, counter reset, one kernel per shape, result copy) is built
 // as a CUDA graph the first time a set of shapes is seen at a given size class and replayed
@@ -36,7 +36,8 @@ struct Group {
     CUfunction fn;
     int grid, threads;
     size_t smem;
-    std::vector<int> work;  // flattened {query, unit} pairs
+    std::vector<int> work;  // {query, first unit} pairs
+    long long units;
 };
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -190,7 +191,7 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
         auto f = gid.find(it.plan->batch_fn);
         if (f == gid.end()) {
             gid[it.plan->batch_fn] = (int)groups.size();
-            groups.push_back({it.plan->batch_fn, it.plan->batch_grid, it.plan->batch_threads, it.plan->batch_smem, {}});
+            groups.push_back({it.plan->batch_fn, it.plan->batch_grid, it.plan->batch_threads, it.plan->batch_smem, {}, 0});
             f = gid.find(it.plan->batch_fn);
         }
         it.group = f->second;
@@ -217,15 +218,16 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
     if (rc) return rc;
     if (scr != (void*)b->d_scratch) drop_graphs(b);
     b->d_scratch = (unsigned char*)scr;
-    // work lists: per group [count, pad, pairs...]
+    // work lists: per group [units, queries, {query, first unit}...]
     std::vector<size_t> goff(groups.size());
     size_t words = 0;
     for (size_t i = 0; i < n; i++) {
         auto& it = b->items[i];
-        for (int u = 0; u < it.units; u++) {
-            groups[it.group].work.push_back((int)i);
-            groups[it.group].work.push_back(u);
-        }
+        Group& g = groups[it.group];
+        if (g.units + it.units > 0x7fffffffLL) return fail(ctx, RF_ERR_INVALID, "batch has too many work units");
+        g.work.push_back((int)i);
+        g.work.push_back((int)g.units);
+        g.units += it.units;
     }
     for (size_t g = 0; g < groups.size(); g++) {
         goff[g] = words;
@@ -241,8 +243,8 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
     b->h_work = (int*)hw;
     for (size_t g = 0; g < groups.size(); g++) {
         int* p = b->h_work + goff[g];
-        p[0] = (int)(groups[g].work.size() / 2);
-        p[1] = 0;
+        p[0] = (int)groups[g].units;
+        p[1] = (int)(groups[g].work.size() / 2);
         std::memcpy(p + 2, groups[g].work.data(), groups[g].work.size() * 4);
     }
     // parameter blocks point into the batch's scratch
@@ -266,7 +268,7 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
     std::string sig = std::to_string(ncls) + ":" + std::to_string(b->out_bytes);
     for (size_t g = 0; g < groups.size(); g++)
         sig += "|" + std::to_string((uintptr_t)groups[g].fn) + "@" + std::to_string(goff[g]) + "/" +
-               std::to_string(size_class(groups[g].work.size() / 2));
+               std::to_string(size_class(groups[g].work.size() / 2)) + "*" + std::to_string(size_class((size_t)groups[g].units));
     auto gi = b->graphs.find(sig);
     if (gi == b->graphs.end()) {
         // built node by node (no stream capture, which would interact with other threads'
@@ -292,13 +294,12 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
         CUresult cr = CUDA_SUCCESS;
         for (size_t g = 0; g < groups.size() && e == cudaSuccess && cr == CUDA_SUCCESS; g++) {
             const RfParams* pp = b->d_params;
-            const int* wl = b->d_work + goff[g] + 2;
-            const int* nw = b->d_work + goff[g];
-            void* kargs[] = {&pp, &wl, &nw};
+            const int* wl = b->d_work + goff[g];
+            void* kargs[] = {&pp, &wl};
             CUDA_KERNEL_NODE_PARAMS kp{};
             kp.func = groups[g].fn;
             int cap = std::max(1, groups[g].grid * b->share_pct / 100);
-            kp.gridDimX = (unsigned)std::max(1, std::min(cap, (int)size_class(groups[g].work.size() / 2)));
+            kp.gridDimX = (unsigned)std::max(1, std::min(cap, (int)std::min<size_t>(size_class((size_t)groups[g].units), 1 << 30)));
             kp.gridDimY = kp.gridDimZ = 1;
             kp.blockDimX = (unsigned)groups[g].threads;
             kp.blockDimY = kp.blockDimZ = 1;

@@ -381,11 +381,98 @@ RF_DEV bool rf_df_step(float2 a, double v, float2& out)
     return ok;
 }
 
-// the double nearest hi + lo of a double-float slot, as slot bits
-RF_DEV unsigned long long rf_df_slot_to_f64(unsigned long long w)
+// Two slots of neighbouring aggregates at once, for addends in the split's range (Z: or +0; checked
+// before, rf_df_in and rf_df_ok).  The low float is rounded here, not truncated: |v - (hi + lo)| is at
+// most 2^-47 v and has no bias, which pays for the few double-float additions that fold the threads'
+// slots (rf_df_add_df2).  The slots are kept as one float4 {hi0, hi1, lo0, lo1}, so that one 16-byte access
+// moves both and their high and low parts are register pairs for Blackwell's two-wide FP32
+// instructions (add.f32x2, sub.f32x2): the same additions, correctly rounded, in half the instructions.
+RF_DEV bool rf_df_in(double v) { return (unsigned)__double2hiint(v) - (920u << 20) < (194u << 20); }
+
+RF_DEV bool rf_df_ok(double v) { return rf_df_in(v) || __double_as_longlong(v) == 0; }
+
+template <bool Z>
+RF_DEV void rf_df_split_in(double v, float& hi, float& lo)
 {
-    const double hi = (double)__uint_as_float((unsigned)w), lo = (double)__uint_as_float((unsigned)(w >> 32));
-    return rf_f2u(__dadd_rn(hi, lo));
+    const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+    const unsigned hb = __funnelshift_l(l, h - (896u << 20), 3);  // as in rf_df_split
+    const unsigned c = (hb & 0x7F800000u) - (23u << 23);
+    hi = __uint_as_float(Z && h == 0u ? 0u : hb);
+    lo = __uint_as_float(c + (((l & 0x1FFFFFFFu) + 32u) >> 6)) - __uint_as_float(c);  // 0 for +0
+}
+
+RF_DEV unsigned long long rf_f2(float x, float y)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+RF_DEV void rf_unf2(unsigned long long v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+RF_DEV unsigned long long rf_add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+RF_DEV unsigned long long rf_sub2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// two pairs += two pairs {hi0, hi1, lo0, lo1}, non-negative (rf_df_add_same_sign, two wide)
+RF_DEV void rf_df_add_df2(float4& a, const float4& b)
+{
+    unsigned long long ah = rf_f2(a.x, a.y), al = rf_f2(a.z, a.w);
+    const unsigned long long bh = rf_f2(b.x, b.y), bl = rf_f2(b.z, b.w);
+    const unsigned long long s = rf_add2(ah, bh), bb = rf_sub2(s, ah);
+    unsigned long long e = rf_add2(rf_sub2(ah, rf_sub2(s, bb)), rf_sub2(bh, bb));
+    e = rf_add2(e, rf_add2(al, bl));
+    ah = rf_add2(s, e);
+    al = rf_sub2(e, rf_sub2(ah, s));
+    rf_unf2(ah, a.x, a.y);
+    rf_unf2(al, a.z, a.w);
+}
+
+template <bool Z>
+RF_DEV void rf_df_add_pair(float4& a, double v0, double v1)
+{
+    float h0, l0, h1, l1;
+    rf_df_split_in<Z>(v0, h0, l0);
+    rf_df_split_in<Z>(v1, h1, l1);
+    rf_df_add_df2(a, make_float4(h0, h1, l0, l1));
+}
+
+template <bool Z>
+RF_DEV void rf_df_add_one(float2& a, double v)
+{
+    float bh, bl;
+    rf_df_split_in<Z>(v, bh, bl);
+    rf_df_add_same_sign(a.x, a.y, bh, bl);
+}
+
+// A double-float slot as an integer, in units of 2^(eh - 179) where eh is hi's biased exponent: 53 bits
+// hold hi exactly and lo, at most half a unit of hi's last place, rounded.  hi is 0 or a normal float
+// of 2^-103 and above; lo is scaled by two powers of two that are floats (exactly) and converted.
+RF_DEV unsigned long long rf_df_int(float hi, float lo)
+{
+    const unsigned hb = __float_as_uint(hi), eh = hb >> 23;
+    const bool small = eh < 64u;
+    const float s1 = small ? 0x1p60f : 1.f, s2 = __uint_as_float((306u - eh - (small ? 60u : 0u)) << 23);
+    const unsigned long long m = (unsigned long long)((hb & 0x7FFFFFu) | 0x800000u) << 29;
+    return hb ? m + (unsigned long long)(long long)__float2int_rn(__fmul_rn(__fmul_rn(lo, s1), s2)) : 0ULL;
+}
+
+// The double nearest hi + lo of a double-float slot, as slot bits, with integer instructions only.
+RF_DEV unsigned long long rf_df_to_f64(float hi, float lo)
+{
+    const unsigned hb = __float_as_uint(hi);
+    unsigned long long m = rf_df_int(hi, lo);
+    if (m == 0) return 0ULL;
+    int E = (int)(hb >> 23) - 127 + 1023;
+    if (!(m >> 52)) m <<= 1, E--;
+    return ((unsigned long long)E << 52) + (m - (1ULL << 52));
 }
 
 // ---------------------------------------------------------------------------------------

@@ -10,6 +10,24 @@
 #define RF_FOLD_ACC 4
 #endif
 
+// Batched form: one persistent launch runs the work units of many queries of this shape.  work
+// names the shape's queries and where their units begin: work[0] = {units, queries}, then per query
+// {index of its parameter block, its first unit}, in unit order; a block finds the query of its
+// next unit by bisection.  (A list of every unit, 15 000 of them for 64 queries, took the host and
+// its copy longer than the kernels.)  A query's units are the ones its stand-alone launch would run,
+// folded in the same order: same bits either way.
+RF_DEV int2 rf_batch_unit(const int2* work, int w)
+{
+    int lo = 0, hi = work[0].y;  // the last query whose first unit is not after w
+    while (hi - lo > 1) {
+        const int m = (lo + hi) >> 1;
+        if (__ldg(&work[1 + m].y) <= w) lo = m;
+        else hi = m;
+    }
+    const int2 q = __ldg(work + 1 + lo);
+    return make_int2(q.x, w - q.y);
+}
+
 // ---------------------------------------------------------------------------------------
 // Template 1: fused scan-filter-project-reduce.
 //   The fragment defines: struct RfAcc (8-byte aligned fields, size a multiple of 8),
@@ -117,9 +135,6 @@ RF_DEV void rf_scan_reduce_merge(const RfParams& P, int unit, int nunits, RfAcc&
     __syncthreads();  // shared state is reused by the next work item of a persistent block
 }
 
-// Batched form: one persistent launch runs the work units of many queries of this shape.
-// work[w] = {query, unit}; params[query] is the query's parameter block.  A query's units are
-// the ones its stand-alone launch would run, folded in the same order: same bits either way.
 #define RF_SCAN_REDUCE_KERNEL(NAME, T)                                                      \
     extern "C" __global__ void __launch_bounds__(T) NAME(const __grid_constant__ RfParams P) \
     {                                                                                       \
@@ -129,11 +144,11 @@ RF_DEV void rf_scan_reduce_merge(const RfParams& P, int unit, int nunits, RfAcc&
         rf_scan_reduce_merge<T>(P, P.unit0 + (int)blockIdx.x, P.nunits, acc);               \
     }                                                                                       \
     extern "C" __global__ void __launch_bounds__(T)                                         \
-        rf_batch(const RfParams* __restrict__ params, const int2* __restrict__ work, const int* nwork) \
+        rf_batch(const RfParams* __restrict__ params, const int2* __restrict__ work)       \
     {                                                                                       \
-        const int n = *nwork;                                                               \
+        const int n = work[0].x;                                                            \
         for (int w = blockIdx.x; w < n; w += gridDim.x) {                                   \
-            const int2 it = work[w];                                                        \
+            const int2 it = rf_batch_unit(work, w);                                         \
             const RfParams& Q = params[it.x];                                               \
             if (it.y < 0 || it.y >= Q.nunits) { /* a malformed work item: report, skip */  \
                 if (threadIdx.x == 0) atomicExch(Q.err, RF_DEVERR_RANGE);                    \
@@ -151,13 +166,18 @@ RF_DEV void rf_scan_reduce_merge(const RfParams& P, int unit, int nunits, RfAcc&
 // Template 2: grouped scan-reduce with shared-memory privatised accumulators.
 //   The fragment defines RF_G groups x RF_M aggregates, struct RfVals, rf_group(P, r, V)
 //   (group id or -1, and the row's aggregate inputs), rf_slot_init(m) (64-bit identity),
-//   rf_slot_combine(m, a, b), rf_slot_add(S, g, t, V, df), rf_slots_done(S, t, df) (df: the
-//   thread keeps its FP64 sums as double-floats, see rf_device.cuh) and
-//   rf_finish_groups(P, tot, out).  With RF_GROUP_SPLIT it also defines the row's loads apart,
+//   rf_slot_combine(m, a, b), rf_slot_at(q, t) (where thread t keeps slot q: S[q * T + t], or side
+//   by side with its neighbour's), rf_slot_add(S, g, t, V, df), rf_slots_done(S, t, df) (df: the
+//   thread keeps its FP64 sums as double-floats, see rf_device.cuh; RF_GROUP_DF: it can, and
+//   rf_slot_kind(m) - 1: alone, 2: with the next slot, 3: with the one before -, rf_slot_df(S, q, t,
+//   kind) {hi, hi of the next, lo, lo of the next} and rf_df_task(i), the RF_DF_TASKS aggregates of
+//   kinds 1 and 2, read them) and
+//   rf_finish_groups(P, tot, out, part, parts) (the output fields part, part + parts, ...).  With RF_GROUP_SPLIT it also defines the row's loads apart,
 //   struct RfRowLd, rf_group_ld(P, r, L) and rf_group_v(P, r, L, V) (rf_group is the two in turn).
-// Each thread owns a private column of G*M 64-bit slots in shared memory (slot (q, t) at
-// S[q * T + t]): no atomics and no bank conflicts on the per-row update.  At the end every
-// slot column is folded over the block in a fixed order, then over units by the last unit.
+// Each thread owns a private column of G*M 64-bit slots in shared memory: no atomics and no bank
+// conflicts on the per-row update.  At the end every slot column is folded over the block in a fixed
+// order, then over units by the last unit, whose warps compute the output fields between them (a
+// field may divide, and one thread doing all 18 quotients of the 6-group group-by in turn took 6 us).
 // ---------------------------------------------------------------------------------------
 #ifdef RF_GROUP_REDUCE
 template <int T>
@@ -167,7 +187,7 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
     __shared__ int last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Q = RF_G * RF_M;
-    for (int q = 0; q < Q; q++) S[q * T + tid] = rf_slot_init(P, q % RF_M);
+    for (int q = 0; q < Q; q++) S[rf_slot_at(q, tid)] = rf_slot_init(P, q % RF_M);
     bool df = true;  // the thread's FP64 sum slots hold double-floats (rf_slot_add, rf_slots_done)
     long long lo = P.row_lo, hi = P.row_hi;
     if (P.range) {
@@ -266,13 +286,53 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
 #endif
 #endif
     }
-    rf_slots_done(S, tid, df);
+#ifdef RF_GROUP_DF
+    const bool sums_df = __syncthreads_and(df) != 0;  // every thread's FP64 sums are still double-floats
+    if (!sums_df) {
+        rf_slots_done(S, tid, df);
+        __syncthreads();
+    }
+#else
     __syncthreads();
+#endif
     unsigned long long* part = (unsigned long long*)P.partials;
+#ifdef RF_GROUP_DF
+    // Double-floats are folded as they are (each is the sum of many such additions already), two
+    // neighbouring slots at once, and turned into doubles last: a conversion and an addition of doubles
+    // for each thread's slot hold the FP64 pipe for 16 cycles a warp each.  (The fold of 36 slots of
+    // 512 threads: 34K cycles with doubles, 9K so with one chain of additions a warp, 4K with four.)
+    if (sums_df)
+        for (int i = warp; i < RF_G * RF_DF_TASKS; i += T / 32) {
+            const int q = i / RF_DF_TASKS * RF_M + rf_df_task(i % RF_DF_TASKS), kind = rf_slot_kind(q % RF_M);
+            constexpr int C = T / 32 < 4 ? T / 32 : 4;
+            float4 a[C];
+#pragma unroll
+            for (int k = 0; k < C; k++) a[k] = rf_slot_df(S, q, lane + 32 * k, kind);
+#pragma unroll
+            for (int k = C; k < T / 32; k++) rf_df_add_df2(a[k % C], rf_slot_df(S, q, lane + 32 * k, kind));
+#pragma unroll
+            for (int w = C / 2; w > 0; w >>= 1)
+#pragma unroll
+                for (int k = 0; k < w; k++) rf_df_add_df2(a[k], a[k + w]);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+                rf_df_add_df2(a[0], make_float4(__shfl_down_sync(0xffffffffu, a[0].x, off), __shfl_down_sync(0xffffffffu, a[0].y, off),
+                                                __shfl_down_sync(0xffffffffu, a[0].z, off), __shfl_down_sync(0xffffffffu, a[0].w, off)));
+            if (lane == 0) {
+                __stcg(part + (long long)unit * Q + q, rf_df_to_f64(a[0].x, a[0].z));
+                if (kind == 2) __stcg(part + (long long)unit * Q + q + 1, rf_df_to_f64(a[0].y, a[0].w));
+            }
+        }
+    // the other slots, from the last warp on (the first ones have most of the tasks above)
+    for (int q = T / 32 - 1 - warp; q < Q; q += T / 32) {
+        const int m = q % RF_M;
+        if (sums_df && rf_slot_kind(m)) continue;
+#else
     for (int q = warp; q < Q; q += T / 32) {
         const int m = q % RF_M;
-        unsigned long long a = S[q * T + lane];
-        for (int k = 1; k < T / 32; k++) a = rf_slot_combine(m, a, S[q * T + lane + 32 * k]);
+#endif
+        unsigned long long a = S[rf_slot_at(q, lane)];
+        for (int k = 1; k < T / 32; k++) a = rf_slot_combine(m, a, S[rf_slot_at(q, lane + 32 * k)]);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) a = rf_slot_combine(m, a, __shfl_down_sync(0xffffffffu, a, off));
         if (lane == 0) __stcg(part + (long long)unit * Q + q, a);
@@ -291,6 +351,18 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
             // units lane, lane+32, ... folded in that order; their loads are issued RF_FOLD at a
             // time ahead of the combines
             unsigned long long a = rf_slot_init(P, m);
+#ifdef RF_GROUP_DF
+            // (few units, large blocks: the last loads go out together too)
+            for (int u = lane; u - lane < nunits; u += 32 * 8) {
+                unsigned long long v[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (u + 32 * k < nunits) v[k] = __ldcg(part + (long long)(u + 32 * k) * Q + q);
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (u + 32 * k < nunits) a = rf_slot_combine(m, a, v[k]);
+            }
+#else
             int u = lane;
             for (; u + 32 * (RF_FOLD - 1) < nunits; u += 32 * RF_FOLD) {
                 unsigned long long v[RF_FOLD];
@@ -300,15 +372,15 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
                 for (int k = 0; k < RF_FOLD; k++) a = rf_slot_combine(m, a, v[k]);
             }
             for (; u < nunits; u += 32) a = rf_slot_combine(m, a, __ldcg(part + (long long)u * Q + q));
+#endif
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) a = rf_slot_combine(m, a, __shfl_down_sync(0xffffffffu, a, off));
             if (lane == 0) S[q] = a;
         }
         __syncthreads();
-        if (tid == 0) {
-            rf_finish_groups(P, S, P.out);
-            *P.counter = 0u;
-        }
+        // neighbouring fields to different warps, which then differ in what they compute
+        rf_finish_groups(P, S, P.out, lane * (T / 32) + warp, T);
+        if (tid == 0) *P.counter = 0u;
     }
     __syncthreads();  // shared state is reused by the next work item of a persistent block
 }
@@ -327,11 +399,11 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
         rf_group_reduce<T>(P, P.unit0 + (int)blockIdx.x, P.nunits);                         \
     }                                                                                       \
     extern "C" __global__ void RF_GROUP_BOUNDS(T)                                           \
-        rf_batch(const RfParams* __restrict__ params, const int2* __restrict__ work, const int* nwork) \
+        rf_batch(const RfParams* __restrict__ params, const int2* __restrict__ work)       \
     {                                                                                       \
-        const int n = *nwork;                                                               \
+        const int n = work[0].x;                                                            \
         for (int w = blockIdx.x; w < n; w += gridDim.x) {                                   \
-            const int2 it = work[w];                                                        \
+            const int2 it = rf_batch_unit(work, w);                                         \
             if (it.y < 0 || it.y >= params[it.x].nunits) { /* malformed work item */       \
                 if (threadIdx.x == 0) atomicExch(params[it.x].err, RF_DEVERR_RANGE);         \
                 continue;                                                                   \

@@ -2020,38 +2020,103 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
                 if (use_df && lf.op == AggOp::SUM && !lf.count && lf.type.btype == FLOAT64) dfm.push_back(m);
             }
             if (!dfm.empty()) so << "#define RF_GROUP_UNROLL 1\n\n";
-            so << "RF_DEV void rf_slots_done(unsigned long long* S, int t, bool& df)\n{\n";
-            if (!dfm.empty()) {
-                so << "    if (!df) return;\n    df = false;\n    for (int g = 0; g < RF_G; g++) {\n";
-                for (int m : dfm)
-                    so << "        { unsigned long long* s = S + (g * RF_M + " << m << ") * " << T
-                      << " + t; *s = rf_df_slot_to_f64(*s); }\n";
+            // double-float slots of neighbouring aggregates share one float4 per thread (rf_df_add_pair)
+            std::vector<int> first_of_pair;
+            for (size_t i = 0; i + 1 < dfm.size(); i++)
+                if (dfm[i + 1] == dfm[i] + 1) first_of_pair.push_back(dfm[i++]);
+            auto paired = [&](int m) {  // the pair's first aggregate, or -1
+                for (int f : first_of_pair)
+                    if (m == f || m == f + 1) return f;
+                return -1;
+            };
+            const std::string Ts = std::to_string(T);
+            so << "RF_DEV int rf_slot_at(int q, int t)\n{\n";
+            if (!first_of_pair.empty()) {
+                so << "    switch (q % RF_M) {\n";
+                for (int f : first_of_pair)
+                    so << "        case " << f << ": return q * " << Ts << " + 2 * t;\n        case " << f + 1 << ": return (q - 1) * " << Ts
+                       << " + 2 * t + 1;\n";
                 so << "    }\n";
-            } else {
-                so << "    (void)S; (void)t; (void)df;\n";
             }
-            so << "}\n\n";
-            so << "RF_DEV void rf_slot_add(unsigned long long* S, int g, int t, const RfVals& V, bool& df)\n{\n";
+            so << "    return q * " << Ts << " + t;\n}\n\n";
             auto slot_ptr = [&](int m) {
-                return "S + (g * RF_M + " + std::to_string(m) + ") * " + std::to_string(T) + " + t";
+                const int f = paired(m);
+                if (f < 0) return "S + (g * RF_M + " + std::to_string(m) + ") * " + Ts + " + t";
+                return "S + (g * RF_M + " + std::to_string(f) + ") * " + Ts + " + 2 * t" + (m == f ? "" : " + 1");
             };
             if (!dfm.empty()) {
-                // every double-float slot of the row in one pass (independent latency chains), one
-                // combined check, then all stores - or the switch to FP64 for the rest of the unit
-                so << "    bool fp64 = !df;\n    if (df) {\n        bool ok = true;\n";
+                so << "#define RF_GROUP_DF 1\nRF_DEV int rf_slot_kind(int m)\n{\n    switch (m) {\n";
                 for (int m : dfm)
-                    so << "        float2* p" << m << " = (float2*)(" << slot_ptr(m) << ");\n        float2 n" << m << ";\n";
-                for (int m : dfm) so << "        ok &= rf_df_step(*p" << m << ", V.v" << m << ", n" << m << ");\n";
-                so << "        if (ok) {\n";
-                for (int m : dfm) so << "            *p" << m << " = n" << m << ";\n";
-                so << "        } else {\n            rf_slots_done(S, t, df);\n            fp64 = true;\n        }\n    }\n";
-                so << "    if (fp64) {\n";
+                    so << "        case " << m << ": return " << (paired(m) < 0 ? 1 : paired(m) == m ? 2 : 3) << ";\n";
+                so << "        default: return 0;\n    }\n}\n\n"
+                      "RF_DEV int rf_df_task(int i)\n{\n    switch (i) {\n";
+                int tasks = 0;
+                for (int m : dfm)
+                    if (paired(m) < 0 || paired(m) == m) so << "        case " << tasks++ << ": return " << m << ";\n";
+                so << "        default: return 0;\n    }\n}\n#define RF_DF_TASKS " << tasks << "\n\n"
+                      "RF_DEV float4 rf_slot_df(const unsigned long long* S, int q, int t, int kind)\n{\n"
+                      "    if (kind == 2) return *(const float4*)(S + (q * " << Ts << " + 2 * t));\n"
+                      "    const float2 a = *(const float2*)(S + (q * " << Ts << " + t));\n    return make_float4(a.x, 0.f, a.y, 0.f);\n}\n\n";
+                so << "static __device__ __noinline__ void rf_slots_to_f64(unsigned long long* S, int t)\n{\n    for (int g = 0; g < RF_G; g++) {\n";
+                for (int m : dfm) {
+                    if (paired(m) >= 0 && paired(m) != m) continue;
+                    if (paired(m) == m)
+                        so << "        { ulonglong2* s = (ulonglong2*)(" << slot_ptr(m) << "); const float4 a = *(float4*)s; "
+                           << "*s = make_ulonglong2(rf_df_to_f64(a.x, a.z), rf_df_to_f64(a.y, a.w)); }\n";
+                    else
+                        so << "        { unsigned long long* s = " << slot_ptr(m) << "; const float2 a = *(float2*)s; *s = rf_df_to_f64(a.x, a.y); }\n";
+                }
+                so << "    }\n}\n\n";
+            }
+            so << "RF_DEV void rf_slots_done(unsigned long long* S, int t, bool& df)\n{\n";
+            if (!dfm.empty()) so << "    if (df) rf_slots_to_f64(S, t);\n    df = false;\n}\n\n";
+            else so << "    (void)S; (void)t; (void)df;\n}\n\n";
+            if (!dfm.empty()) {
+                // the row's addends onto its slots; Z: some of them are zeros
+                auto add = [&](const std::string& ind, const std::string& v, const char* Z) {
+                    auto ty = [&](int m) { return std::string(paired(m) == m ? "float4" : "float2"); };
+                    for (int m : dfm) {
+                        if (paired(m) >= 0 && paired(m) != m) continue;
+                        const std::string k = std::to_string(m);
+                        so << ind << ty(m) << "* p" << k << " = (" << ty(m) << "*)(" << slot_ptr(m) << ");\n" << ind << ty(m) << " a" << k << " = *p"
+                           << k << ";\n";
+                    }
+                    for (int m : dfm) {
+                        if (paired(m) >= 0 && paired(m) != m) continue;
+                        if (paired(m) == m)
+                            so << ind << "rf_df_add_pair<" << Z << ">(a" << m << ", " << v << m << ", " << v << m + 1 << ");\n";
+                        else
+                            so << ind << "rf_df_add_one<" << Z << ">(a" << m << ", " << v << m << ");\n";
+                    }
+                    for (int m : dfm)
+                        if (paired(m) < 0 || paired(m) == m) so << ind << "*p" << m << " = a" << m << ";\n";
+                };
+                // a warp with an addend that is zero, negative or out of the double-float range: a zero
+                // adds nothing; anything else turns the thread's slots into doubles for the rest of the
+                // unit.  A function of its own, so that the loop's code stays small: four rows of it are
+                // fetched cold by every launch (a 1000-row group-by spends most of its time on that).
+                so << "static __device__ __noinline__ bool rf_slot_add_some(unsigned long long* S, int g, int t, bool df";
+                for (int m : dfm) so << ", double v" << m;
+                so << ")\n{\n    if (df";
+                for (int m : dfm) so << " && rf_df_ok(v" << m << ")";
+                so << ") {\n";
+                add("        ", "v", "true");
+                so << "        return true;\n    }\n    if (df) rf_slots_to_f64(S, t);\n";
                 for (int m : dfm) {
                     auto& lf = leaves[g0[m]];
-                    so << "        { unsigned long long* s = " << slot_ptr(m) << "; *s = rf_slot_combine(" << m << ", *s, "
-                      << enc(lf, "V.v" + std::to_string(m)) << "); }\n";
+                    so << "    { unsigned long long* s = " << slot_ptr(m) << "; *s = rf_slot_combine(" << m << ", *s, "
+                      << enc(lf, "v" + std::to_string(m)) << "); }\n";
                 }
-                so << "    }\n";
+                so << "    return false;\n}\n\n";
+                so << "RF_DEV void rf_slot_add(unsigned long long* S, int g, int t, const RfVals& V, bool& df)\n{\n    const bool in = df";
+                for (int m : dfm) so << " & rf_df_in(V.v" << m << ")";
+                so << ";\n    if (__all_sync(__activemask(), in)) {\n";
+                add("        ", "V.v", "false");
+                so << "    } else {\n        df = rf_slot_add_some(S, g, t, df";
+                for (int m : dfm) so << ", V.v" << m;
+                so << ");\n    }\n";
+            } else {
+                so << "RF_DEV void rf_slot_add(unsigned long long* S, int g, int t, const RfVals& V, bool& df)\n{\n";
             }
             for (int m = 0; m < M; m++) {
                 if (std::find(dfm.begin(), dfm.end(), m) != dfm.end()) continue;
@@ -2245,9 +2310,43 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         }
         std::ostringstream stores;
         emit_output_store(Ef, stores, red, finals);
-        o << "RF_DEV void rf_finish_groups(const RfParams& P, const unsigned long long* S, unsigned char* out)\n{\n";
-        for (auto& dcl : Ef.decls) o << "    " << dcl << "\n";
-        o << fb.str() << stores.str() << "}\n\n";
+        // one case per output field, with the final states it reads; shared declarations (an output that
+        // reads tables, say) leave all fields to one thread
+        std::ostringstream fdecl;
+        for (auto& dcl : Ef.decls) fdecl << "    " << dcl << "\n";
+        std::vector<std::string> fields;
+        {
+            std::istringstream in(stores.str());
+            std::string line;
+            while (std::getline(in, line)) fields.push_back(line);
+        }
+        bool apart = Ef.decls.empty();
+        for (auto& f : fields) apart = apart && f.compare(0, 6, "    *(") == 0;
+        o << "RF_DEV void rf_finish_groups(const RfParams& P, const unsigned long long* S, unsigned char* out, int part, int parts)\n{\n";
+        if (!apart) {
+            o << "    if (part != 0) return;\n" << fdecl.str() << fb.str() << stores.str() << "}\n\n";
+        } else {
+            o << "    for (int f = part; f < " << fields.size() << "; f += parts) {\n        switch (f) {\n";
+            for (size_t f = 0; f < fields.size(); f++) {
+                o << "        case " << f << ": {\n";
+                std::istringstream in(fb.str());
+                std::string line;
+                while (std::getline(in, line)) {
+                    // "    const T stK = ...;": kept where the field names stK
+                    const size_t at = line.find(" st"), eq = line.find(" = ");
+                    if (at == std::string::npos || eq == std::string::npos || at > eq) continue;
+                    const std::string nm = line.substr(at + 1, eq - at - 1);
+                    for (size_t p = fields[f].find(nm); p != std::string::npos; p = fields[f].find(nm, p + 1)) {
+                        const char nx = p + nm.size() < fields[f].size() ? fields[f][p + nm.size()] : ' ';
+                        if (isdigit((unsigned char)nx)) continue;
+                        o << "        " << line << "\n";
+                        break;
+                    }
+                }
+                o << "        " << fields[f] << "\n            break;\n        }\n";
+            }
+            o << "        }\n    }\n}\n\n";
+        }
 
         src << o.str();
         size_t smem = (size_t)G * M * T * 8 + (compact ? (size_t)(T / 32) * 64 * 8 : 0);
@@ -2265,6 +2364,12 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         src << "RF_GROUP_REDUCE_KERNEL(rf_main, " << T << ")\n";
         plan_.kernels.push_back({"rf_main", T, smem, KernelSpec::MAIN});
         plan_.acc_bytes = (size_t)G * M * 8;
+        plan_.compact = compact;
+        // Double-float sums run faster in blocks of 512 threads, where their slots fit one: the rows of a
+        // step are held in 104 registers a thread instead of 80 (the 6-group group-by, each at its best
+        // tile: 60M rows 548 us against 591 us at 256 threads, 6M 84 / 107, 1M 37 / 47, 100K 29 / 29)
+        const size_t smem512 = (size_t)G * M * 512 * 8;
+        if (!compact && o.str().find("rf_slots_to_f64") != std::string::npos && smem512 <= 200 * 1024) plan_.pref_threads = 512;
     }
 
     // ---------------------------------------------------------------- Op lowering (tables)

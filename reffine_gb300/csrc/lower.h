@@ -90,6 +90,8 @@ struct Plan {
     int hg_hot = 0;                     // hash group-by: hottest keys folded per warp (index 2x)
     int hg_warm = 0;                    // hash group-by: further hot keys in shared memory (index 2x)
     int groups = 0, aggs = 0;           // grouped plans
+    bool compact = false;               // grouped plans: rows are queued before their index probe
+    int pref_threads = 256;             // the block size the plan runs fastest at, untuned
     std::vector<DataType> out_cols;     // table outputs: column types
     int out_dim = 0;
     bool vectorize = false;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import loopgen
-from parity import assert_table_same
+from parity import assert_same, assert_table_same
 from reffine_gb300.ir import _add, _func, _get, _gt, _i64, _in, _lt, _op, _sym, _i64_t
 from reffine_gb300.table import Table
 from test_gpu_materialize import plan_run_table
@@ -89,3 +89,22 @@ def test_merges_at_tile_edges(eng, name, mode, vectorize):
             np.testing.assert_array_equal(g[v], r[w])
     else:
         assert_table_same(out, ref)
+
+
+@pytest.mark.parametrize("ncol", [1, 2, 3, 5])
+@pytest.mark.parametrize("zeros", [0.0, 0.1, 1.0])
+def test_grouped_sums_with_zeros_at_tile_edges(eng, zeros, ncol):
+    # one to five double-float sums (alone and in pairs); zero addends leave the fast path, one
+    # negative addend at the end turns a thread's slots into doubles
+    from widequery import wide_groupby_query, wide_table
+    for n in (1, 511, 4095, 4096, 4097, 70_001):
+        for negative in (False, True):
+            t = wide_table(n, ncol, seed=n)
+            rng = np.random.default_rng(n + ncol)
+            for c in t.columns[3:]:
+                c.data[rng.random(n) < zeros] = 0.0
+                if negative:
+                    c.data[-1] = -1.5
+            fn = wide_groupby_query(t.get_data_type(), ncol)
+            got = eng.compile(fn).run(eng.upload(t))
+            assert_same(got, loopgen.Query(fn)(t))
