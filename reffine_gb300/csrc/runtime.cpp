@@ -1116,16 +1116,18 @@ extern "C" int rf_plan_compile(rf_ctx* ctx, const char* text, int vectorize, rf_
     cudaSetDevice(ctx->device);
     std::shared_ptr<reffine::Func> fn;
     std::string shape;
+    int threads = 256;
     try {
         fn = reffine::parse_text(text);
-        shape = rfg::lower(fn, vectorize != 0).key;  // the query shape at the default block size
+        const rfg::Plan l = rfg::lower(fn, vectorize != 0);
+        shape = l.key;  // the query shape, named at 256 threads
+        threads = l.pref_threads;
     } catch (const rfg::LowerError& e) {
         return fail(ctx, e.unsupported ? RF_ERR_UNSUPPORTED : RF_ERR_INVALID, "%s", e.what());
     } catch (const std::exception& e) {
         return fail(ctx, RF_ERR_INVALID, "%s", e.what());
     }
     // a block size the autotuner chose for this shape (kept as bucket -1 of the shape's entry)
-    int threads = 256;
     {
         std::lock_guard<std::mutex> g(ctx->tune_mu);
         auto it = ctx->tune.find(shape);
@@ -1248,6 +1250,37 @@ int hg_factor_for(rf_plan* p, long long rows)
     return jt == it->second.end() ? 220 : (int)jt->second;
 }
 
+// The tiling of a scan that was not tuned: tiles that give the resident blocks the same number of
+// rows, so that no last wave is partly filled and a small table uses the whole GPU (8192-row tiles
+// left 2 blocks for 10K rows, 123 for 1M, and 17 tiles to some units and 16 to others at 60M).
+long long untuned_tile_rows(rf_plan* p, long long rows)
+{
+    const rfg::Plan& pl = p->plan;
+    const long long T = pl.threads, wave = std::max(1, p->max_units), sms = std::max(1, p->ctx->sm_count);
+    auto up = [](long long x, long long m) { return (std::max(x, 1LL) + m - 1) / m * m; };
+    auto share = [&](long long units) { return (std::max(rows, 1LL) + units - 1) / units; };
+    if (pl.kind == rfg::PlanKind::SCAN_REDUCE) {
+        // one unit to a resident block; a table of less than 4096 rows to each takes about two units an
+        // SM, of two 4-row steps of their threads at least (filter+sum, 8192-row tiles / these: 10K rows
+        // 13.3 / 8.2 us, 100K 14.4 / 8.3, 1M 15.2 / 12.3, 6M 45.3 / 34.2, 50M 216 / 207)
+        return std::max(up(share(wave), 4), 4096LL);
+    }
+    if (pl.compact) {
+        // rows cost very different amounts (the ones that reach the probe), and those may lie together
+        // in a sorted table: four waves of units even them out where each has 8192 rows; a smaller table
+        // is spread over fewer units.  Whole steps of 8 rows a thread.  (join probes, 8192-row tiles /
+        // these: 100K rows 34 / 17 us, 3M 41 / 33, 20M 135 / 135, 200M 1218 / 1090; 200M sorted by
+        // the filter's column 1159 / 1098, where one wave takes 4158 us and two 2062)
+        const long long small = std::min(8192LL, std::max(share(wave), 4096LL));
+        return up(std::max(share(4 * wave), small), 8 * T);
+    }
+    // one tile to a unit: its threads then step through whole blocks of rows to the end, and rows enough
+    // are in flight without a prefetch (6-group group-by of 512 threads, 8192-row tiles / 4096-row
+    // tiles, each prefetched while the one before is summed / these: 1M rows 28 / 29 / 27 us, 6M 77 / 74 /
+    // 73, 20M 211 / 200 / 189, 60M 543 / 537 / 518); two 4-row steps of its threads at least
+    return std::max(8 * T, up(share(wave), 32));
+}
+
 long long tile_rows_for(rf_plan* p, long long rows)
 {
     const rfg::Plan& pl = p->plan;
@@ -1257,9 +1290,9 @@ long long tile_rows_for(rf_plan* p, long long rows)
     while (bucket < 62 && (1LL << (bucket + 1)) <= rows) bucket++;
     std::lock_guard<std::mutex> g(p->ctx->tune_mu);
     auto it = p->ctx->tune.find(pl.key);
-    if (it == p->ctx->tune.end()) return pl.tile_rows;
+    if (it == p->ctx->tune.end()) return untuned_tile_rows(p, rows);
     auto jt = it->second.find(bucket);
-    return jt == it->second.end() ? pl.tile_rows : jt->second;
+    return jt == it->second.end() ? untuned_tile_rows(p, rows) : jt->second;
 }
 
 int fill_params(rf_plan* p, const rf_arg* args, int n_args, RfParams& P, long long& lo, long long& hi,
@@ -1547,6 +1580,9 @@ int run_streamed(rf_plan* p, const rf_arg* args, int n_args, const std::vector<H
         if (fill_params(p, args, n_args, P0, lo0, hi0, true) == RF_OK) {
             const int u = units_for(p, (hi0 - lo0 + P0.tile_rows - 1) / P0.tile_rows);
             nchunks = std::min(kChunks, u / std::max(1, ctx->sm_count));
+            // (one unit an SM, as large blocks have: two halves, so that the first runs while the second
+            // is copied)
+            if (nchunks == 1 && u >= ctx->sm_count) nchunks = 2;
         }
     }
     if (nchunks < 2) pinned = false;
@@ -1765,6 +1801,10 @@ int tune_tiles(rf_plan* p, const rf_arg* args, int32_t n_args, int32_t reps, int
         const long long units = (long long)p->max_units * w;
         const long long t = ((rows + units - 1) / units + 3) & ~3LL;
         if (t >= 256 && t <= 65536 && std::find(cand.begin(), cand.end(), t) == cand.end()) cand.push_back(t);
+    }
+    {
+        const long long t = untuned_tile_rows(p, rows);
+        if (std::find(cand.begin(), cand.end(), t) == cand.end()) cand.push_back(t);
     }
     // each timing runs k launches back to back (k such that they take about 2 ms: a short kernel
     // timed alone is mostly launch latency and its jitter), as a query stream runs them; the

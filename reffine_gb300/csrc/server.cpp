@@ -74,7 +74,8 @@ size_t footprint_of(rf_plan* p, long long lo, long long hi)
     const rfg::Plan& pl = p->plan;
     long long rows = std::max<long long>(hi - lo, 0);
     if (!pl.out_is_table) {
-        long long ntiles = (rows + pl.tile_rows - 1) / pl.tile_rows;
+        const long long tile = rfrt::tile_rows_for(p, rows);
+        long long ntiles = (rows + tile - 1) / tile;
         long long units = units_for(p, ntiles);
         return (size_t)units * pl.acc_bytes + 2 * std::max<size_t>(pl.out_size, 16) + sizeof(RfParams);
     }
