@@ -2293,7 +2293,7 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         Emitter Ef(*this);
         bind_inputs(Ef);
         std::map<std::vector<size_t>, std::string> finals;
-        std::ostringstream fb;
+        std::vector<std::string> states;  // "const T stK = ...;" of leaf K
         std::map<int, std::pair<int, int>> leaf_gm;
         for (int g = 0; g < G; g++)
             for (int m = 0; m < M; m++) leaf_gm[groups[g][m]] = {g, m};
@@ -2305,7 +2305,7 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
                 tot = dec(lf, "S[" + std::to_string(gm.first * M + gm.second) + "]");
             }
             std::string nm = "st" + std::to_string(i);
-            fb << "    const " << ctype(lf.type) << " " << nm << " = " << final_leaf(Ef, lf, tot) << ";\n";
+            states.push_back("    const " + ctype(lf.type) + " " + nm + " = " + final_leaf(Ef, lf, tot) + ";\n");
             finals[lf.path] = nm;
         }
         std::ostringstream stores;
@@ -2324,25 +2324,20 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         for (auto& f : fields) apart = apart && f.compare(0, 6, "    *(") == 0;
         o << "RF_DEV void rf_finish_groups(const RfParams& P, const unsigned long long* S, unsigned char* out, int part, int parts)\n{\n";
         if (!apart) {
-            o << "    if (part != 0) return;\n" << fdecl.str() << fb.str() << stores.str() << "}\n\n";
+            o << "    if (part != 0) return;\n" << fdecl.str();
+            for (auto& st : states) o << st;
+            o << stores.str() << "}\n\n";
         } else {
             o << "    for (int f = part; f < " << fields.size() << "; f += parts) {\n        switch (f) {\n";
             for (size_t f = 0; f < fields.size(); f++) {
                 o << "        case " << f << ": {\n";
-                std::istringstream in(fb.str());
-                std::string line;
-                while (std::getline(in, line)) {
-                    // "    const T stK = ...;": kept where the field names stK
-                    const size_t at = line.find(" st"), eq = line.find(" = ");
-                    if (at == std::string::npos || eq == std::string::npos || at > eq) continue;
-                    const std::string nm = line.substr(at + 1, eq - at - 1);
-                    for (size_t p = fields[f].find(nm); p != std::string::npos; p = fields[f].find(nm, p + 1)) {
-                        const char nx = p + nm.size() < fields[f].size() ? fields[f][p + nm.size()] : ' ';
-                        if (isdigit((unsigned char)nx)) continue;
-                        o << "        " << line << "\n";
-                        break;
-                    }
+                std::set<size_t> used;  // the states stK that the field names
+                for (size_t p = fields[f].find("st"); p != std::string::npos; p = fields[f].find("st", p + 2)) {
+                    const char* d = fields[f].c_str() + p + 2;
+                    if (isdigit((unsigned char)*d)) used.insert(std::min((size_t)strtoul(d, nullptr, 10), states.size()));
                 }
+                for (size_t k : used)
+                    if (k < states.size()) o << "        " << states[k];
                 o << "        " << fields[f] << "\n            break;\n        }\n";
             }
             o << "        }\n    }\n}\n\n";
