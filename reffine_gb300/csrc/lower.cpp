@@ -2497,15 +2497,18 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
     // unsorted.  The groups are the distinct valid keys - the runs the reference would see after
     // sorting and run-end encoding - so each output row is the same; rows come out in slot order.
     //   rf_hg_init  fills the table: keys RF_EMPTY_KEY, accumulators at their identity
-    //   rf_hg_agg   one pass over the rows.  A per-block shared-memory table takes the keys a
-    //               block meets first - under a skewed distribution the frequent ones - and
-    //               absorbs their updates with shared-memory atomics; a key found neither there
-    //               nor in a free shared slot goes to the global open-addressing table (load 0.5)
+    //   rf_hg_agg   one pass over the rows: those of the hottest keys fold inside their warp, the others
+    //               go to the global open-addressing table with atomics
     //   rf_cond / rf_emit   the materialisation template over the slots
-    // Global slots are array-of-structs, {key, accumulators...} padded to RF_HG_SW 8-byte words
-    // (one 32-byte sector for up to three accumulators), so a row touches one sector.
-    // Device layout: slots (unsigned long long*)P.aux4 [C + 1][RF_HG_SW] (slot C: the key
-    // RF_EMPTY_KEY itself, a used flag in its key word), rows P.aux_n0, capacity C = P.aux_n1.
+    // The global table is two arrays (one for wide rows, see `joint`): the slots' keys, and their accumulators padded to RF_HG_AS words.
+    // Probing is linear from the first slot of a 32-byte sector of four keys, which one step reads
+    // whole: at load 0.45 a key is almost always among them, so the lanes of a warp seldom wait for a
+    // longer chain; found, a row adds to its accumulators without waiting.  (The call over 100M Zipf
+    // rows of 10M keys: 2218 us with slots of {key, accumulators} probed one by one, 2031 with the two
+    // arrays, 1921 with four keys a step.)
+    // Device layout: keys (unsigned long long*)P.aux4 [C + 1] (C a multiple of 4; slot C: the key
+    // RF_EMPTY_KEY itself, a used flag in its key word), from word (C + 8) & ~7 on accumulators
+    // [C + 1][RF_HG_AS]; rows P.aux_n0, capacity C = P.aux_n1.
     // rows per lane in one step of the aggregation loop: with 2 or 4 (all loads and probes of a
     // step issued before any is used) the 100M-row group-by took 3.6 and 5.0 ms against 2.1 ms
     static int hg_rows_per_step() { return 1; }
@@ -2520,8 +2523,6 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         for (size_t i = 0; i < leaves.size(); i++)
             if (leaves[i].op != AggOp::NONE) act.push_back((int)i);
         const int L = (int)act.size();
-        // shared-memory tiers of the aggregation kernel (see rf_hg_agg below): HK hottest keys
-        // with warp-private accumulators, WK further hot keys with block-shared accumulators
         // the aggregation kernel's hottest keys (see rf_hg_agg below): HK keys with warp-private
         // accumulators, at most 16 KB of them per block
         const int HT = 256, HW = HT / 32, LL = std::max(L, 1);
@@ -2533,12 +2534,18 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         std::string c0 = "P.t[" + sl + "].col[0]";
         std::ostringstream o;
         o << "// generated by the reffine_gb300 lowering pass: " << fn_->name << " (hash group-by)\n";
-        const int SW = L + 1 <= 4 ? 4 : (L + 1 <= 8 ? 8 : 16);
+        // Nine to fifteen aggregates keep a slot in one array, {key, accumulators} in one 128-byte line,
+        // probed one by one: the atomics of an update then go to one line (20M Zipf rows of 2M keys, two
+        // arrays against one: 2 aggregates 374 / 457 us, 4 693 / 816, 7 1671 / 1866, 10 3090 / 2985,
+        // 15 4934 / 4192).  In the two arrays a slot's accumulators are whole 16-byte pairs, which span
+        // fewer sectors, but for 3 and 7 of them, which fill a power of two of words with the key's.
+        const bool joint = LL > 8;
+        const int AS = joint ? 15 : LL == 1 || LL == 3 || LL == 7 ? LL : (LL + 1) & ~1;
         if (L + 1 > 16) throw LowerError("hash group-by with more than 15 aggregates");
-        o << "#include \"rf_device.cuh\"\n\n#define RF_HG_L " << LL << "\n#define RF_HG_SW " << SW
-          << "\n#define RF_HG_T " << HT << "\n#define RF_HG_HK " << HK << "\n#define RF_HG_U " << hg_rows_per_step()
+        o << "#include \"rf_device.cuh\"\n\n#define RF_HG_L " << LL << "\n#define RF_HG_AS " << AS
+          << "\n#define RF_HG_JOINT " << (joint ? 1 : 0) << "\n#define RF_HG_T " << HT << "\n#define RF_HG_HK " << HK << "\n#define RF_HG_U " << hg_rows_per_step()
           << "\n#define RF_HG_SPK " << kHotSlotsPerKey << "\n\n";
-        plan_.acc_bytes = (size_t)SW * 8;
+        plan_.acc_bytes = 8 + (size_t)AS * 8;
         auto kind_of = [&](const Leaf& lf) -> std::string {
             bool f = lf.type.is_float() && !lf.count;
             switch (lf.op) {
@@ -2651,18 +2658,81 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
             o << "    " << call << ";\n";
         }
         o << "    (void)A; (void)B; (void)st; (void)bst;\n}\n\n";
-        o << R"(// slot of `key` in the global table from probe position h on (claimed if new): one
-// compare-and-swap per probe, which claims an empty slot or finds the key in one round trip
-// (hot keys never come here, so the slots are not contended)
-RF_DEV long long rf_hg_slot_from(const RfParams& P, long long key, unsigned long long h, unsigned long long n0)
+        o << R"(#if RF_HG_JOINT
+#define RF_HG_NK 1  // keys one probing step reads
+#define RF_HG_KS (1 + RF_HG_AS)  // words from key to key
+#else
+#define RF_HG_NK 4
+#define RF_HG_KS 1
+#endif
+
+// the key word of slot g
+RF_DEV unsigned long long* rf_hg_key(const RfParams& P, unsigned long long g)
 {
-    unsigned long long* tab = (unsigned long long*)P.aux4;
-    const unsigned long long C = (unsigned long long)P.aux_n1;
-    for (unsigned long long n = 0; n < n0; ++n) {
-        const unsigned long long old =
-            atomicCAS(tab + h * RF_HG_SW, (unsigned long long)RF_EMPTY_KEY, (unsigned long long)key);
-        if (old == (unsigned long long)RF_EMPTY_KEY || old == (unsigned long long)key) return (long long)h;
-        if (++h == C) h = 0;
+    return (unsigned long long*)P.aux4 + g * RF_HG_KS;
+}
+
+// the accumulators of slot g
+RF_DEV unsigned long long* rf_hg_acc(const RfParams& P, long long g)
+{
+#if RF_HG_JOINT
+    return rf_hg_key(P, g) + 1;
+#else
+    return (unsigned long long*)P.aux4 + ((P.aux_n1 + 8) & ~7LL) + g * RF_HG_AS;
+#endif
+}
+
+// the slot a key's probing starts from
+RF_DEV unsigned long long rf_hg_home(long long key, unsigned long long C)
+{
+    return RF_HG_NK * rf_home(key, C / RF_HG_NK);
+}
+
+struct RfHgKeys {
+    unsigned long long k[RF_HG_NK];
+};
+
+// the keys of one probing step from slot h on, through L1: a claimed slot's key never changes, and a
+// stale empty is corrected by the compare-and-swap
+RF_DEV RfHgKeys rf_hg_keys(const RfParams& P, unsigned long long h)
+{
+    RfHgKeys s;
+#if RF_HG_JOINT
+    s.k[0] = __ldca(rf_hg_key(P, h));
+#else
+    const ulonglong2* p = (const ulonglong2*)rf_hg_key(P, h);
+    const ulonglong2 a = __ldca(p), b = __ldca(p + 1);
+    s.k[0] = a.x, s.k[1] = a.y, s.k[2] = b.x, s.k[3] = b.y;
+#endif
+    return s;
+}
+
+// place of `key` among a step's keys, RF_HG_NK when it is not there
+RF_DEV int rf_hg_among(const RfHgKeys& s, unsigned long long key)
+{
+    int f = RF_HG_NK;
+#pragma unroll
+    for (int i = RF_HG_NK - 1; i >= 0; i--)
+        if (s.k[i] == key) f = i;
+    return f;
+}
+
+// slot of `key` in the global table (claimed if new) given the keys from its home slot h on; slots
+// are taken in probing order, by one compare-and-swap each, which claims an empty slot or finds the
+// key in one round trip (hot keys never come here, so the slots are not contended)
+RF_DEV long long rf_hg_slot_from(const RfParams& P, long long key, unsigned long long h, RfHgKeys s)
+{
+    const unsigned long long C = (unsigned long long)P.aux_n1, kw = (unsigned long long)key;
+    for (unsigned long long n = 0; n < C; n += RF_HG_NK) {
+        const int f = rf_hg_among(s, kw);
+        if (f < RF_HG_NK) return (long long)h + f;
+        for (int i = rf_hg_among(s, (unsigned long long)RF_EMPTY_KEY); i < RF_HG_NK; i++) {
+            const unsigned long long old = atomicCAS(rf_hg_key(P, h + i), (unsigned long long)RF_EMPTY_KEY, kw);
+            if (old == (unsigned long long)RF_EMPTY_KEY || old == kw) return (long long)h + i;
+        }
+        h += RF_HG_NK;
+        if (h >= C) h = 0;
+        s = rf_hg_keys(P, h);
     }
     rf_set_err(P, RF_DEVERR_OVERFLOW);
     return -1;
@@ -2671,37 +2741,44 @@ RF_DEV long long rf_hg_slot_from(const RfParams& P, long long key, unsigned long
 // slot of `key` in the global table (claimed if new); C + 1 slots, slot C is the empty key's
 RF_DEV long long rf_hg_slot(const RfParams& P, long long key)
 {
-    unsigned long long* tab = (unsigned long long*)P.aux4;
     const unsigned long long C = (unsigned long long)P.aux_n1;
     if (key == RF_EMPTY_KEY) {
-        if (tab[C * RF_HG_SW] == 0) atomicExch(tab + C * RF_HG_SW, 1ULL);
+        if (*rf_hg_key(P, C) == 0) atomicExch(rf_hg_key(P, C), 1ULL);
         return (long long)C;
     }
-    return rf_hg_slot_from(P, key, rf_home(key, C), C);
+    const unsigned long long h = rf_hg_home(key, C);
+    return rf_hg_slot_from(P, key, h, rf_hg_keys(P, h));
 }
 
 extern "C" __global__ void __launch_bounds__(256) rf_hg_init(const __grid_constant__ RfParams P)
 {
-    unsigned long long* tab = (unsigned long long*)P.aux4;
     const long long C = P.aux_n1;
     // word by word, so a warp's stores are contiguous
-    const long long words = (C + 1) * RF_HG_SW;
-    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < words; w += (long long)gridDim.x * blockDim.x) {
-        const long long s = w / RF_HG_SW;
-        const int f = (int)(w % RF_HG_SW);
-        tab[w] = f == 0 ? (s < C ? (unsigned long long)RF_EMPTY_KEY : 0ULL)
-                        : (f <= RF_HG_L ? rf_hg_identity(P, f - 1) : 0ULL);
+    const long long stride = (long long)gridDim.x * blockDim.x, w0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+#if RF_HG_JOINT
+    unsigned long long* tab = rf_hg_key(P, 0);
+    for (long long w = w0; w < (C + 1) * RF_HG_KS; w += stride) {
+        const long long g = w / RF_HG_KS;
+        const int f = (int)(w % RF_HG_KS) - 1;
+        tab[w] = f >= 0 ? (f < RF_HG_L ? rf_hg_identity(P, f) : 0ULL) : g < C ? (unsigned long long)RF_EMPTY_KEY : 0ULL;
     }
+#else
+    unsigned long long* keys = rf_hg_key(P, 0);
+    unsigned long long* acc = rf_hg_acc(P, 0);
+    for (long long w = w0; w <= C; w += stride) keys[w] = w < C ? (unsigned long long)RF_EMPTY_KEY : 0ULL;
+    for (long long w = w0; w < (C + 1) * RF_HG_AS; w += stride) {
+        const int f = (int)(w % RF_HG_AS);
+        acc[w] = f < RF_HG_L ? rf_hg_identity(P, f) : 0ULL;
+    }
+#endif
 }
 
 // Aggregation.  Rows of the hottest keys (chosen from a sample of the key column, so Zipf-like
 // skew lands here) fold inside each warp: the lanes holding the same hot key find each other
 // with __match_any_sync, the lowest of them folds their contributions and adds them, without
 // atomics, to the warp's own accumulators.  All other rows go to the global table, whose
-// accumulators take fire-and-forget atomics; its keys are read through L1 first (a claimed
-// slot's key never changes; a stale empty is corrected by the compare-and-swap).  The hot-key
-// index is a read-only table built on the host: open addressing, load <= 0.5, 32-bit
-// multiplicative hash of the folded key.
+// accumulators take fire-and-forget atomics.  The hot-key index is a read-only table built on the
+// host: open addressing, load <= 0.5, 32-bit multiplicative hash of the folded key.
 // The hot-key table is collision-free (the host chose its hash multiplier and left out any key
 // whose slot a hotter key took), so a lookup is one probe.
 // Dynamic shared memory:
@@ -2711,24 +2788,6 @@ RF_DEV unsigned rf_hg_h32(long long key, unsigned mult, int bits)
 {
     const unsigned f = (unsigned)key ^ (unsigned)((unsigned long long)key >> 32);
     return (f * mult) >> (32 - bits);
-}
-
-RF_DEV long long rf_hg_slot_l1(const RfParams& P, long long key, unsigned long long h, unsigned long long n0)
-{
-    unsigned long long* tab = (unsigned long long*)P.aux4;
-    const unsigned long long C = (unsigned long long)P.aux_n1;
-    for (unsigned long long n = 0; n < n0; ++n) {
-        unsigned long long* kp = tab + h * RF_HG_SW;
-        const unsigned long long cur = __ldca(kp);
-        if (cur == (unsigned long long)key) return (long long)h;
-        if (cur == (unsigned long long)RF_EMPTY_KEY) {
-            const unsigned long long old = atomicCAS(kp, (unsigned long long)RF_EMPTY_KEY, (unsigned long long)key);
-            if (old == (unsigned long long)RF_EMPTY_KEY || old == (unsigned long long)key) return (long long)h;
-        }
-        if (++h == C) h = 0;
-    }
-    rf_set_err(P, RF_DEVERR_OVERFLOW);
-    return -1;
 }
 
 extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_constant__ RfParams P)
@@ -2753,7 +2812,6 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
     for (int i = tid; i < W * RF_HG_HK * RF_HG_L; i += RF_HG_T) wacc[i] = rf_hg_identity(P, i % RF_HG_L);
     for (int i = tid; i < RF_HG_HK; i += RF_HG_T) seen[i] = 0;
     __syncthreads();
-    unsigned long long* tab = (unsigned long long*)P.aux4;
     unsigned long long* wa = wacc + (size_t)warp * RF_HG_HK * RF_HG_L;
     unsigned long long* x = xs + ((size_t)warp * 32 + lane) * RF_HG_L;
     unsigned long long top[RF_HG_L];  // the lane's sums of hot id 0
@@ -2786,15 +2844,15 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
             const unsigned q = rf_hg_h32(key[j], mult, bits);
             h[j] = act[j] && key[j] != RF_EMPTY_KEY && hk[q] == key[j] ? (int)hid[q] : -1;
         }
-        // first read of each cold row's home slot, issued for all the step's rows at once
-        unsigned long long home[RF_HG_U], first[RF_HG_U];
+        // the first read of each cold row's probing, issued for all the step's rows at once
+        unsigned long long home[RF_HG_U];
+        RfHgKeys first[RF_HG_U];
 #pragma unroll
         for (int j = 0; j < RF_HG_U; j++) {
             home[j] = 0;
-            first[j] = (unsigned long long)RF_EMPTY_KEY;
             if (act[j] && h[j] < 0 && key[j] != RF_EMPTY_KEY) {
-                home[j] = rf_home(key[j], C);
-                first[j] = __ldca(tab + home[j] * RF_HG_SW);
+                home[j] = rf_hg_home(key[j], C);
+                first[j] = rf_hg_keys(P, home[j]);
             }
         }
 #pragma unroll
@@ -2841,22 +2899,8 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
 #pragma unroll
         for (int j = 0; j < RF_HG_U; j++) {
             if (!act[j] || h[j] >= 0) continue;
-            long long g;
-            if (key[j] == RF_EMPTY_KEY) {
-                g = rf_hg_slot(P, key[j]);
-            } else if (first[j] == (unsigned long long)key[j]) {
-                g = (long long)home[j];
-            } else {
-                // the home slot is empty (claim it) or holds another key: probe on from the next
-                g = -1;
-                if (first[j] == (unsigned long long)RF_EMPTY_KEY) {
-                    const unsigned long long old = atomicCAS(tab + home[j] * RF_HG_SW, (unsigned long long)RF_EMPTY_KEY,
-                                                             (unsigned long long)key[j]);
-                    if (old == (unsigned long long)RF_EMPTY_KEY || old == (unsigned long long)key[j]) g = (long long)home[j];
-                }
-                if (g < 0) g = rf_hg_slot_l1(P, key[j], home[j] + 1 == C ? 0 : home[j] + 1, C - 1);
-            }
-            if (g >= 0) rf_hg_apply(P, row[j], tab + g * RF_HG_SW + 1, 1);
+            const long long g = key[j] == RF_EMPTY_KEY ? rf_hg_slot(P, key[j]) : rf_hg_slot_from(P, key[j], home[j], first[j]);
+            if (g >= 0) rf_hg_apply(P, row[j], rf_hg_acc(P, g), 1);
         }
     }
     // the lanes' sums of hot id 0 into their warp's accumulator of it
@@ -2883,24 +2927,24 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
 #pragma unroll
             for (int l = 0; l < RF_HG_L; l++) a[l] = rf_hg_comb(l, a[l], wacc[((size_t)w2 * RF_HG_HK + id) * RF_HG_L + l]);
         const long long g = rf_hg_slot(P, hk[i]);
-        if (g >= 0) rf_hg_merge(P, tab + g * RF_HG_SW + 1, 1, a, 1);
+        if (g >= 0) rf_hg_merge(P, rf_hg_acc(P, g), 1, a, 1);
     }
 }
 
 )";
         // element functions over the slots
         auto elem = [&](Emitter& E, std::ostringstream& body) {
-            body << "    const unsigned long long* sl = (const unsigned long long*)P.aux4 + r * RF_HG_SW;\n";
-            body << "    const long long C = P.aux_n1;\n";
-            body << "    const bool used = r < C ? (long long)sl[0] != RF_EMPTY_KEY : sl[0] != 0;\n";
-            body << "    const int64_t it = r < C ? (long long)sl[0] : RF_EMPTY_KEY;\n";
+            body << "    const unsigned long long* sl = rf_hg_acc(P, r);\n";
+            body << "    const long long C = P.aux_n1, kw = (long long)*rf_hg_key(P, r);\n";
+            body << "    const bool used = r < C ? kw != RF_EMPTY_KEY : kw != 0;\n";
+            body << "    const int64_t it = r < C ? kw : RF_EMPTY_KEY;\n    (void)sl;\n";
             E.bind(op.iters[0], E.scalar("it", d.sp.iter->type));
             std::map<std::vector<size_t>, std::string> finals;
             for (size_t i = 0, k = 0; i < leaves.size(); i++) {
                 auto& lf = leaves[i];
                 std::string tot = "0";
                 if (lf.op != AggOp::NONE) {
-                    std::string raw = "sl[" + std::to_string(k + 1) + "]";
+                    std::string raw = "sl[" + std::to_string(k) + "]";
                     tot = (lf.type.is_float() && !lf.count) ? "rf_u2f(" + raw + ")" : "(long long)(" + raw + ")";
                     k++;
                 }

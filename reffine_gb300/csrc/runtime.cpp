@@ -2195,11 +2195,12 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         const int factor = hg_factor_for(p, vt->cols[0].logical);
         hg_cap = std::max<long long>(1024, (long long)((double)factor / 100.0 * (double)ndv));
         if (p->hg_retry_cap > hg_cap) hg_cap = p->hg_retry_cap;
-        // slots of pl.acc_bytes bytes: {key, accumulators} (array of structs).  The table is
+        hg_cap = (hg_cap + 3) & ~3LL;  // whole sectors of keys
+        // slots of pl.acc_bytes bytes: keys, accumulators (and up to 64 bytes between).  The table is
         // taken from the pool for this run and handed back when the run ends (stream-ordered):
         // a serving mix holds thousands of hash group-by plans (one per query's constants), and
         // each keeping its table measured 52 GB for 722 plans.
-        if (!grow(&p->hg_keys, &p->hg_keys_cap, (size_t)(hg_cap + 1) * pl.acc_bytes, s))
+        if (!grow(&p->hg_keys, &p->hg_keys_cap, (size_t)(hg_cap + 1) * pl.acc_bytes + 64, s))
             return fail(ctx, RF_ERR_OOM, "hash table allocation (%lld slots)", hg_cap);
         P.aux4 = p->hg_keys;
         P.aux_n0 = vt->cols[0].logical;

@@ -5,7 +5,7 @@ import pytest
 
 from oracle import loopgen
 from parity import assert_same, assert_table_same
-from reffine_gb300.ir import _add, _func, _get, _gt, _i64, _in, _lt, _op, _sym, _i64_t
+from reffine_gb300.ir import _add, _f64, _func, _get, _gt, _i64, _in, _lt, _new, _op, _red, _sym, _i64_t
 from reffine_gb300.table import Table
 from test_gpu_materialize import plan_run_table
 
@@ -108,3 +108,36 @@ def test_grouped_sums_with_zeros_at_tile_edges(eng, zeros, ncol):
             fn = wide_groupby_query(t.get_data_type(), ncol)
             got = eng.compile(fn).run(eng.upload(t))
             assert_same(got, loopgen.Query(fn)(t))
+
+
+@pytest.mark.parametrize("nsum", [0, 1, 2, 3, 4, 5, 6, 9, 12])
+@pytest.mark.parametrize("n,nkeys", [(1, 1), (700, 460), (5000, 4999), (70_001, 30_000)])
+def test_hash_group_by_slots(eng, n, nkeys, nsum):
+    # every width of a slot's accumulators; keys that overflow their sector of four, and the key that
+    # marks an empty slot.  Whole-number values: sums are exact
+    rng = np.random.default_rng(n + nsum)
+    keys = rng.integers(-2**62, 2**62, nkeys)
+    keys[-1] = np.iinfo(np.int64).min
+    cols = {"key": keys[rng.integers(0, nkeys, n)]}
+    for i in range(nsum):
+        cols["v%d" % i] = rng.integers(-1000, 1000, n).astype(np.float64)
+    if nsum == 0:
+        cols["v"] = np.zeros(n)
+    t = Table.from_arrays(2, cols, name="slots")
+    vec, k = _sym("vec", t.get_data_type()), _sym("k", _i64_t)
+    red = _red(vec[k], lambda: _new([_f64(0)] * nsum + [_i64(0)]),
+               lambda s, v: _new([_add(_get(s, i), _get(v, i)) for i in range(nsum)] + [_add(_get(s, nsum), _i64(1))]))
+    rs = _sym("agg", red)
+    op = _op([k], _in(k, vec), [_get(rs, i) for i in range(nsum + 1)])
+    os_ = _sym("op", op)
+    fn = _func("slots", os_, [vec])
+    fn.tbl[rs], fn.tbl[os_] = red, op
+    plan = eng.compile(fn)
+    assert plan.kind == 5
+    out = plan_run_table(eng, plan, t)
+    order = np.argsort(out["cols"][0], kind="stable")
+    uk, inv = np.unique(cols["key"], return_inverse=True)
+    np.testing.assert_array_equal(out["cols"][0][order], uk)
+    for i in range(nsum):
+        np.testing.assert_array_equal(out["cols"][1 + i][order], np.bincount(inv, weights=cols["v%d" % i], minlength=len(uk)))
+    np.testing.assert_array_equal(out["cols"][1 + nsum][order], np.bincount(inv, minlength=len(uk)))
