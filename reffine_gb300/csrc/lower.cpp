@@ -2543,7 +2543,7 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         const int AS = joint ? 15 : LL == 1 || LL == 3 || LL == 7 ? LL : (LL + 1) & ~1;
         if (L + 1 > 16) throw LowerError("hash group-by with more than 15 aggregates");
         o << "#include \"rf_device.cuh\"\n\n#define RF_HG_L " << LL << "\n#define RF_HG_AS " << AS
-          << "\n#define RF_HG_JOINT " << (joint ? 1 : 0) << "\n#define RF_HG_T " << HT << "\n#define RF_HG_HK " << HK << "\n#define RF_HG_U " << hg_rows_per_step()
+          << "\n#define RF_HG_JOINT " << (joint ? 1 : 0)  << "\n#define RF_HG_T " << HT << "\n#define RF_HG_HK " << HK << "\n#define RF_HG_U " << hg_rows_per_step()
           << "\n#define RF_HG_SPK " << kHotSlotsPerKey << "\n\n";
         plan_.acc_bytes = 8 + (size_t)AS * 8;
         auto kind_of = [&](const Leaf& lf) -> std::string {
@@ -2858,42 +2858,37 @@ extern "C" __global__ void __launch_bounds__(RF_HG_T) rf_hg_agg(const __grid_con
 #pragma unroll
         for (int j = 0; j < RF_HG_U; j++) {
             // the hottest key (hot id 0, about a tenth of the rows under Zipf(1.1)) adds into the
-            // lane's own registers: no fold, and the other hot keys' folds stay short
-            if (h[j] == 0) {
-                unsigned long long xr[RF_HG_L];
-                rf_hg_vals(P, row[j], xr);
+            // lane's own registers, which keeps the folds of the others short; lanes of another hot
+            // key find each other, the lowest folds their values in turn and adds the sum to the
+            // warp's accumulators.  All these last adds are one instruction of the warp, since the
+            // FP64 pipe takes 16 cycles for each, however few its lanes (100M Zipf rows, the call:
+            // 1913 us with an add each for hot id 0, keys alone in the warp and folded ones, 1858
+            // so; 2038 with registers for the two hottest, whose blocks are fewer.  Of 20M rows: 4 aggregates
+            // 686 -> 655 us, 8 2020 -> 1865, 15 4166 -> 3925)
+            const int t = h[j];
+            const unsigned peers = __match_any_sync(0xffffffffu, t >= 1 ? t : -1 - lane);
+            if (t >= 0) rf_hg_vals(P, row[j], x);
+            __syncwarp();
+            unsigned long long xr[RF_HG_L];
 #pragma unroll
-                for (int l = 0; l < RF_HG_L; l++) top[l] = rf_hg_comb(l, top[l], xr[l]);
-                top_seen = true;
+            for (int l = 0; l < RF_HG_L; l++) xr[l] = x[l];
+            const bool lead = t >= 1 && lane == __ffs(peers) - 1;
+            for (unsigned m = lead ? peers & (peers - 1) : 0u; m; m &= m - 1) {
+                const unsigned long long* y = xs + ((size_t)warp * 32 + (__ffs(m) - 1)) * RF_HG_L;
+#pragma unroll
+                for (int l = 0; l < RF_HG_L; l++) xr[l] = rf_hg_comb(l, xr[l], y[l]);
             }
-            // fold of the other hottest keys: lanes of one hot key find each other, the lowest
-            // folds; a key alone in the warp adds straight into the warp's accumulators
-            const unsigned peers = __match_any_sync(0xffffffffu, h[j] >= 1 ? h[j] : -1 - lane);
-            if (h[j] >= 1 && peers == (1u << lane)) {
-                unsigned long long xr[RF_HG_L];
-                rf_hg_vals(P, row[j], xr);
-                unsigned long long* A = wa + (size_t)h[j] * RF_HG_L;
+            __syncwarp();
+            if (lead || t == 0) {
+                unsigned long long* A = wa + (size_t)t * RF_HG_L;
 #pragma unroll
-                for (int l = 0; l < RF_HG_L; l++) A[l] = rf_hg_comb(l, A[l], xr[l]);
-                seen[h[j]] = 1;
-            } else if (h[j] >= 1) {
-                rf_hg_vals(P, row[j], x);
-                __syncwarp(peers);
-                if (lane == __ffs(peers) - 1) {
-                    unsigned long long a[RF_HG_L];
-#pragma unroll
-                    for (int l = 0; l < RF_HG_L; l++) a[l] = x[l];
-                    for (unsigned m = peers & (peers - 1); m; m &= m - 1) {
-                        const unsigned long long* y = xs + ((size_t)warp * 32 + (__ffs(m) - 1)) * RF_HG_L;
-#pragma unroll
-                        for (int l = 0; l < RF_HG_L; l++) a[l] = rf_hg_comb(l, a[l], y[l]);
-                    }
-                    unsigned long long* A = wa + (size_t)h[j] * RF_HG_L;
-#pragma unroll
-                    for (int l = 0; l < RF_HG_L; l++) A[l] = rf_hg_comb(l, A[l], a[l]);
-                    seen[h[j]] = 1;
+                for (int l = 0; l < RF_HG_L; l++) {
+                    const unsigned long long v = rf_hg_comb(l, lead ? A[l] : top[l], xr[l]);
+                    if (lead) A[l] = v;
+                    else top[l] = v;
                 }
-                __syncwarp(peers);
+                if (lead) seen[t] = 1;
+                else top_seen = true;
             }
         }
 #pragma unroll
