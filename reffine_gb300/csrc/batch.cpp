@@ -58,7 +58,7 @@ struct rf_batch {
     std::vector<rf_plan*> groups_plan;
     // device buffers
     RfParams* d_params = nullptr;
-    int* d_work = nullptr;      // per group: [count][pairs...], at group offsets
+    int* d_work = nullptr;      // per group: [units, queries, units taken, 0][pairs...], at group offsets
     unsigned char* d_scratch = nullptr;
     size_t work_cap = 0, scratch_cap = 0;
     // pinned host mirrors
@@ -218,7 +218,7 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
     if (rc) return rc;
     if (scr != (void*)b->d_scratch) drop_graphs(b);
     b->d_scratch = (unsigned char*)scr;
-    // work lists: per group [units, queries, {query, first unit}...]
+    // work lists: per group [units, queries, units taken, 0, {query, first unit}...]
     std::vector<size_t> goff(groups.size());
     size_t words = 0;
     for (size_t i = 0; i < n; i++) {
@@ -231,7 +231,7 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
     }
     for (size_t g = 0; g < groups.size(); g++) {
         goff[g] = words;
-        words += 2 + size_class(groups[g].work.size() / 2) * 2;
+        words += 4 + size_class(groups[g].work.size() / 2) * 2;
     }
     void* w = b->d_work;
     if ((rc = grow_dev(ctx, &w, &b->work_cap, words * 4, last, s))) return rc;
@@ -245,7 +245,8 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
         int* p = b->h_work + goff[g];
         p[0] = (int)groups[g].units;
         p[1] = (int)(groups[g].work.size() / 2);
-        std::memcpy(p + 2, groups[g].work.data(), groups[g].work.size() * 4);
+        p[2] = p[3] = 0;  // units taken so far
+        std::memcpy(p + 4, groups[g].work.data(), groups[g].work.size() * 4);
     }
     // parameter blocks point into the batch's scratch
     for (size_t i = 0; i < n; i++) {

@@ -11,21 +11,52 @@
 #endif
 
 // Batched form: one persistent launch runs the work units of many queries of this shape.  work
-// names the shape's queries and where their units begin: work[0] = {units, queries}, then per query
-// {index of its parameter block, its first unit}, in unit order; a block finds the query of its
-// next unit by bisection.  (A list of every unit, 15 000 of them for 64 queries, took the host and
-// its copy longer than the kernels.)  A query's units are the ones its stand-alone launch would run,
-// folded in the same order: same bits either way.
+// names the shape's queries and where their units begin: work[0] = {units, queries}, work[1] =
+// {units taken beyond each block's first, 0}, then per query {index of its parameter block, its
+// first unit}, in unit order; a block finds the query of its next unit by bisection.  (A list of
+// every unit, 15 000 of them for 64 queries, took the host and its copy longer than the kernels.)  A
+// query's units are the ones its stand-alone launch would run, folded in the same order: same bits
+// either way.
+// Blocks take units as they come free: the kernels of a batch's shapes share the SMs, and with every
+// gridDim.x-th unit the blocks that started last, or had the costlier queries, finished alone.  (64
+// queries of three shapes, from the launch to its end: 426 -> 381 us with tables of 1M rows, 96 -> 98
+// of 150K.  Runs of consecutive units, an eighth, a quarter or half of a block's share, took 388, 387
+// and 402 us, and 2264, 2354 and 2675 us with tables of 8M rows against 2217 unit by unit.)  The next
+// unit is asked for before the one at hand is run, which hides the atomic's way.
 RF_DEV int2 rf_batch_unit(const int2* work, int w)
 {
     int lo = 0, hi = work[0].y;  // the last query whose first unit is not after w
     while (hi - lo > 1) {
         const int m = (lo + hi) >> 1;
-        if (__ldg(&work[1 + m].y) <= w) lo = m;
+        if (__ldg(&work[2 + m].y) <= w) lo = m;
         else hi = m;
     }
-    const int2 q = __ldg(work + 1 + lo);
+    const int2 q = __ldg(work + 2 + lo);
     return make_int2(q.x, w - q.y);
+}
+
+// F(parameters, unit) for every unit that this block gets
+template <class F>
+RF_DEV void rf_batch_units(const RfParams* params, int2* work, F f)
+{
+    __shared__ unsigned taken;
+    const unsigned n = (unsigned)work[0].x;
+#pragma unroll 1
+    for (unsigned w = blockIdx.x; w < n;) {
+        unsigned next = 0;
+        if (threadIdx.x == 0) next = atomicAdd((unsigned*)&work[1].x, 1u);
+        const int2 it = rf_batch_unit(work, (int)w);
+        const RfParams& P = params[it.x];
+        if (it.y < 0 || it.y >= P.nunits) {  // a malformed work item: report, skip
+            if (threadIdx.x == 0) atomicExch(P.err, RF_DEVERR_RANGE);
+        } else {
+            f(P, it.y);
+        }
+        if (threadIdx.x == 0) taken = next;
+        __syncthreads();
+        w = gridDim.x + taken;
+        __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -135,6 +166,7 @@ RF_DEV void rf_scan_reduce_merge(const RfParams& P, int unit, int nunits, RfAcc&
     __syncthreads();  // shared state is reused by the next work item of a persistent block
 }
 
+// (rf_batch: the registers for 768 threads an SM, 80 each; left alone the compiler takes 118)
 #define RF_SCAN_REDUCE_KERNEL(NAME, T)                                                      \
     extern "C" __global__ void __launch_bounds__(T) NAME(const __grid_constant__ RfParams P) \
     {                                                                                       \
@@ -143,22 +175,15 @@ RF_DEV void rf_scan_reduce_merge(const RfParams& P, int unit, int nunits, RfAcc&
         rf_scan_reduce_rows<T>(P, P.unit0 + (int)blockIdx.x, P.nunits, acc);                \
         rf_scan_reduce_merge<T>(P, P.unit0 + (int)blockIdx.x, P.nunits, acc);               \
     }                                                                                       \
-    extern "C" __global__ void __launch_bounds__(T)                                         \
-        rf_batch(const RfParams* __restrict__ params, const int2* __restrict__ work)       \
+    extern "C" __global__ void __launch_bounds__(T, T > 768 ? 1 : 768 / T)                  \
+        rf_batch(const RfParams* __restrict__ params, int2* work)                          \
     {                                                                                       \
-        const int n = work[0].x;                                                            \
-        for (int w = blockIdx.x; w < n; w += gridDim.x) {                                   \
-            const int2 it = rf_batch_unit(work, w);                                         \
-            const RfParams& Q = params[it.x];                                               \
-            if (it.y < 0 || it.y >= Q.nunits) { /* a malformed work item: report, skip */  \
-                if (threadIdx.x == 0) atomicExch(Q.err, RF_DEVERR_RANGE);                    \
-                continue;                                                                   \
-            }                                                                               \
+        rf_batch_units(params, work, [](const RfParams& Q, int unit) {                     \
             RfAcc acc;                                                                      \
             rf_acc_init(Q, acc);                                                            \
-            rf_scan_reduce_rows<T>(Q, it.y, Q.nunits, acc);                                 \
-            rf_scan_reduce_merge<T>(Q, it.y, Q.nunits, acc);                                \
-        }                                                                                   \
+            rf_scan_reduce_rows<T>(Q, unit, Q.nunits, acc);                                 \
+            rf_scan_reduce_merge<T>(Q, unit, Q.nunits, acc);                                \
+        });                                                                                 \
     }
 #endif  // RF_SCAN_REDUCE
 
@@ -399,17 +424,11 @@ RF_DEV void rf_group_reduce(const RfParams& P, int unit, int nunits)
         rf_group_reduce<T>(P, P.unit0 + (int)blockIdx.x, P.nunits);                         \
     }                                                                                       \
     extern "C" __global__ void RF_GROUP_BOUNDS(T)                                           \
-        rf_batch(const RfParams* __restrict__ params, const int2* __restrict__ work)       \
+        rf_batch(const RfParams* __restrict__ params, int2* work)                          \
     {                                                                                       \
-        const int n = work[0].x;                                                            \
-        for (int w = blockIdx.x; w < n; w += gridDim.x) {                                   \
-            const int2 it = rf_batch_unit(work, w);                                         \
-            if (it.y < 0 || it.y >= params[it.x].nunits) { /* malformed work item */       \
-                if (threadIdx.x == 0) atomicExch(params[it.x].err, RF_DEVERR_RANGE);         \
-                continue;                                                                   \
-            }                                                                               \
-            rf_group_reduce<T>(params[it.x], it.y, params[it.x].nunits);                    \
-        }                                                                                   \
+        rf_batch_units(params, work, [](const RfParams& Q, int unit) {                     \
+            rf_group_reduce<T>(Q, unit, Q.nunits);                                          \
+        });                                                                                 \
     }
 #endif  // RF_GROUP_REDUCE
 
