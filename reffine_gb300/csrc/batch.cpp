@@ -214,10 +214,10 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
     size_t scratch_need = off;
     void* scr = b->d_scratch;
     cudaStream_t last = b->last_stream ? b->last_stream : s;
+    if (scratch_need > b->scratch_cap) drop_graphs(b);
     int rc = grow_dev(ctx, &scr, &b->scratch_cap, scratch_need, last, s);
-    if (rc) return rc;
-    if (scr != (void*)b->d_scratch) drop_graphs(b);
     b->d_scratch = (unsigned char*)scr;
+    if (rc) return rc;
     // work lists: per group [units, queries, units taken, 0, {query, first unit}...]
     std::vector<size_t> goff(groups.size());
     size_t words = 0;
@@ -233,14 +233,18 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
         goff[g] = words;
         words += 4 + size_class(groups[g].work.size() / 2) * 2;
     }
+    // a graph is dropped before a buffer that it names is released: a new one may come to lie at the
+    // same address, and the graph's copy nodes would still name the memory that went
+    const size_t list_bytes = std::max<size_t>(words * 4, 16384);
+    if (list_bytes > b->work_cap || list_bytes > b->h_work_cap) drop_graphs(b);
     void* w = b->d_work;
-    if ((rc = grow_dev(ctx, &w, &b->work_cap, words * 4, last, s))) return rc;
-    if (w != (void*)b->d_work) drop_graphs(b);
+    rc = grow_dev(ctx, &w, &b->work_cap, list_bytes, last, s);
     b->d_work = (int*)w;
+    if (rc) return rc;
     void* hw = b->h_work;
-    if ((rc = grow_host(ctx, &hw, &b->h_work_cap, words * 4))) return rc;
-    if (hw != (void*)b->h_work) drop_graphs(b);
+    rc = grow_host(ctx, &hw, &b->h_work_cap, list_bytes);
     b->h_work = (int*)hw;
+    if (rc) return rc;
     for (size_t g = 0; g < groups.size(); g++) {
         int* p = b->h_work + goff[g];
         p[0] = (int)groups[g].units;
@@ -262,9 +266,10 @@ extern "C" int rf_batch_launch(rf_batch* b, void* stream)
     b->out_bytes = ncls * os;
     b->counters_bytes = counters_bytes;
     void* ho = b->h_out;
-    if ((rc = grow_host(ctx, &ho, &b->h_out_cap, counters_bytes + b->out_bytes))) return rc;
-    if (ho != (void*)b->h_out) drop_graphs(b);
+    if (counters_bytes + b->out_bytes > b->h_out_cap) drop_graphs(b);
+    rc = grow_host(ctx, &ho, &b->h_out_cap, counters_bytes + b->out_bytes);
     b->h_out = (unsigned char*)ho;
+    if (rc) return rc;
     // graph: signature = shapes + size classes (copies are sized to the class)
     std::string sig = std::to_string(ncls) + ":" + std::to_string(b->out_bytes);
     for (size_t g = 0; g < groups.size(); g++)

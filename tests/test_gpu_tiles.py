@@ -141,3 +141,23 @@ def test_hash_group_by_slots(eng, n, nkeys, nsum):
     for i in range(nsum):
         np.testing.assert_array_equal(out["cols"][1 + i][order], np.bincount(inv, weights=cols["v%d" % i], minlength=len(uk)))
     np.testing.assert_array_equal(out["cols"][1 + nsum][order], np.bincount(inv, minlength=len(uk)))
+
+
+def test_batch_of_growing_sizes_matches_alone(eng):
+    # one batch reused for lists and results that grow and shrink: its buffers move under the graphs
+    # kept for earlier sizes
+    import ctypes
+    from reffine_gb300 import workloads as W
+    from reffine_gb300.engine import Batch
+    t = W.filter_sum_table(5000, seed=5)
+    dt = eng.upload(t)
+    plans = [eng.compile(W.filter_sum_query(t.get_data_type(), day_lo=i, day_hi=900 + i)) for i in range(7)]
+    alone = [p.run(dt) for p in plans]
+    batch = Batch(eng, 512)
+    for n in (1, 2, 1, 3, 5, 9, 2, 20, 60, 1, 150, 5, 400, 2, 400, 1):
+        for i in range(n):
+            batch.add(plans[i % 7], dt)
+        batch.launch()
+        assert batch.wait() == [alone[i % 7] for i in range(n)]
+        batch.reset()
+    batch.free()
