@@ -2500,8 +2500,8 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
     //   rf_hg_agg   one pass over the rows: those of the hottest keys fold inside their warp, the others
     //               go to the global open-addressing table with atomics
     //   rf_cond / rf_emit   the materialisation template over the slots
-    // The global table is two arrays (one for wide rows, see `joint`): the slots' keys, and their accumulators padded to RF_HG_AS words.
-    // Probing is linear from the first slot of a 32-byte sector of four keys, which one step reads
+    // The global table is two arrays (one for wide rows, see `joint`): the slots' keys, and their
+    // accumulators padded to RF_HG_AS words.  Probing is linear from the first slot of a 32-byte sector of four keys, which one step reads
     // whole: at load 0.45 a key is almost always among them, so the lanes of a warp seldom wait for a
     // longer chain; found, a row adds to its accumulators without waiting.  (The call over 100M Zipf
     // rows of 10M keys: 2218 us with slots of {key, accumulators} probed one by one, 2031 with the two
