@@ -1142,10 +1142,11 @@ extern "C" __global__ void __launch_bounds__(RF_SEG_T) rf_seg_reduce(const __gri
     const long long n = rf_seg_runs(P).len;
     const long long total = (n > 0 ? rf_seg_end(P, n - 1) : 0) + n;  // items
     const long long tile = blockIdx.x;
+    if (tile >= P.aux_n1) return;  // bounds tile and tile + 1 are rf_seg_part's
     long long d0 = tile * RF_SEG_M, d1 = d0 + RF_SEG_M;
     if (d0 > total) d0 = total;
     if (d1 > total) d1 = total;
-    const long long xa = __ldg(part + tile), xb = __ldg(part + tile + 1);
+    const long long xa = __ldg(part + tile), xb = __ldg(part + tile + 1);  // within the runs (rf_warp_search)
     // (bounded for columns whose run ends are out of order, too: never more than a tile's)
     int nx = (int)(xb - xa < 0 ? 0 : xb - xa > RF_SEG_M ? RF_SEG_M : xb - xa);
     const long long ra = d0 - xa;

@@ -2355,10 +2355,14 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
             cap = total;
             P.out_rows = total;
         }
+        // a run-end column of no runs has no tiles, and so no tile boundaries for a block to read
+        if (seg_tiles == 0 && (k.role == rfg::KernelSpec::SEGPART || k.role == rfg::KernelSpec::SEGREDUCE ||
+                               k.role == rfg::KernelSpec::SEGFIX))
+            continue;
         int grid = units;
         if (k.role == rfg::KernelSpec::INIT) grid = ctx->sm_count * 8;
         if (k.role == rfg::KernelSpec::SEGPART) grid = (int)(seg_tiles / 8 + 1);  // a warp per tile boundary
-        if (k.role == rfg::KernelSpec::SEGREDUCE) grid = (int)std::max<long long>(seg_tiles, 1);
+        if (k.role == rfg::KernelSpec::SEGREDUCE) grid = (int)seg_tiles;
         if (k.role == rfg::KernelSpec::SEGFIX) grid = 1;
         if (k.role == rfg::KernelSpec::MERGEPART)
             grid = (int)((union_merge ? P.aux_n0 + P.aux_n1 + 1 : ntiles) / 8 + 1);
