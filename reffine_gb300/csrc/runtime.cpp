@@ -1361,7 +1361,8 @@ int fill_params(rf_plan* p, const rf_arg* args, int n_args, RfParams& P, long lo
         rf_table* t = args[pl.drive_input].table;
         bool aligned = true;
         for (int c : pl.cols_read[pl.drive_input]) {
-            if (t->cols[c].nvals < hi) hi = t->cols[c].nvals;
+            // (a run-end grouping's elements are runs; its rows are bounded where its tiles are laid out)
+            if (t->cols[c].nvals < hi && (pl.kind != rfg::PlanKind::SEG_REDUCE || c == 0)) hi = t->cols[c].nvals;
             aligned = aligned && ((uintptr_t)t->cols[c].data & 15) == 0;
         }
         if (lo < 0) lo = 0;
@@ -2280,7 +2281,9 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
         rf_table* vt = args[pl.drive_input].table;
         const long long nruns = vt->cols[0].nvals;
-        const long long nrows = vt->cols[0].logical;
+        long long nrows = vt->cols[0].logical;
+        for (int c : pl.cols_read[pl.drive_input])
+            if (c != 0) nrows = std::min(nrows, vt->cols[c].nvals);
         seg_tiles = (nruns + nrows + pl.seg_items - 1) / pl.seg_items;
         if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(seg_tiles + 1) * 8, s) ||
             !grow(&p->seg_part, &p->seg_part_cap, (size_t)(nruns + seg_tiles + 1) * pl.acc_bytes, s)) {

@@ -37,3 +37,27 @@ def test_no_runs(eng, wide, vectorize):
             assert out["len"] == 0 and all(len(c) == 0 for c in out["cols"])
         else:
             assert_table_same(out, ref)
+
+
+def geometry(wide):
+    """Items of a thread and of a tile of 128 threads: a staged row and its run end share 36 KiB."""
+    row_bytes = 4 + 8 * (3 if wide else 1)
+    k = max(1, min(22, 36 * 1024 // (128 * row_bytes)))
+    return k, 128 * k
+
+
+def lengths(shape, k, tile):
+    # a run takes an item a row and one for its end
+    return {"thread": [k - 2, k - 1, k, k + 1, 1] * 400,
+            "tile": [tile - 2, tile - 1, tile, tile + 1, 1, tile - 1, 2 * tile - 1],
+            "whole": [tile - 1] * 3, "one_over": [tile - 1] * 3 + [0], "one_short": [tile - 1] * 2 + [tile - 2],
+            "one_run": [3 * tile - 1], "one_run_over": [3 * tile], "ends_only": [0] * (2 * tile) + [5]}[shape]
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("shape", ["thread", "tile", "whole", "one_over", "one_short", "one_run", "one_run_over", "ends_only"])
+def test_runs_at_the_kernels_own_edges(eng, shape, wide):
+    t = runs_table(lengths(shape, *geometry(wide)), wide, seed=len(shape))
+    fn = grouped_query(t.get_data_type(), wide)
+    out = plan_run_table(eng, eng.compile(fn), t)
+    assert_table_same(out, loopgen.Query(fn)(t))
