@@ -383,8 +383,7 @@ RF_DEV bool rf_df_step(float2 a, double v, float2& out)
 
 // Two slots of neighbouring aggregates at once, for addends in the split's range (Z: or +0; checked
 // before, rf_df_in and rf_df_ok).  The low float is rounded here, not truncated: |v - (hi + lo)| is at
-// most 2^-47 v and has no bias, which pays for the few double-float additions that fold the threads'
-// slots (rf_df_add_df2).  The slots are kept as one float4 {hi0, hi1, lo0, lo1}, so that one 16-byte access
+// most 2^-47 v and has no bias.  The slots are kept as one float4 {hi0, hi1, lo0, lo1}, so that one 16-byte access
 // moves both and their high and low parts are register pairs for Blackwell's two-wide FP32
 // instructions (add.f32x2, sub.f32x2): the same additions, correctly rounded, in half the instructions.
 RF_DEV bool rf_df_in(double v) { return (unsigned)__double2hiint(v) - (920u << 20) < (194u << 20); }
@@ -452,27 +451,67 @@ RF_DEV void rf_df_add_one(float2& a, double v)
     rf_df_add_same_sign(a.x, a.y, bh, bl);
 }
 
-// A double-float slot as an integer, in units of 2^(eh - 179) where eh is hi's biased exponent: 53 bits
-// hold hi exactly and lo, at most half a unit of hi's last place, rounded.  hi is 0 or a normal float
-// of 2^-103 and above; lo is scaled by two powers of two that are floats (exactly) and converted.
-RF_DEV unsigned long long rf_df_int(float hi, float lo)
+// The sums of two neighbouring slots over threads, each as h + m + l, three floats that are not
+// renormalised: every addition of the high and middle parts keeps its exact rounding error (Knuth's
+// two-sum), and only the errors' errors are rounded.  A thread's slot has up to 48 bits, so whole
+// numbers, say, are exact in it where their sum over a block needs all the 53 of a double: additions
+// of double-floats would round that at 2^-48.  Sums of 512 non-negative slots stay within 2^-58 of the
+// exact sum here, relative to it (11 two-sums deep the middle part is below 2^-20 of the sum and the
+// last below 2^-39), and the double they become is rounded once (rf_tf_to_f64).
+struct RfTf2 {
+    unsigned long long h, m, l;
+};
+
+RF_DEV void rf_two_sum2(unsigned long long a, unsigned long long b, unsigned long long& s, unsigned long long& e)
 {
-    const unsigned hb = __float_as_uint(hi), eh = hb >> 23;
-    const bool small = eh < 64u;
-    const float s1 = small ? 0x1p60f : 1.f, s2 = __uint_as_float((306u - eh - (small ? 60u : 0u)) << 23);
-    const unsigned long long m = (unsigned long long)((hb & 0x7FFFFFu) | 0x800000u) << 29;
-    return hb ? m + (unsigned long long)(long long)__float2int_rn(__fmul_rn(__fmul_rn(lo, s1), s2)) : 0ULL;
+    s = rf_add2(a, b);
+    const unsigned long long bb = rf_sub2(s, a);
+    e = rf_add2(rf_sub2(a, rf_sub2(s, bb)), rf_sub2(b, bb));
 }
 
-// The double nearest hi + lo of a double-float slot, as slot bits, with integer instructions only.
-RF_DEV unsigned long long rf_df_to_f64(float hi, float lo)
+// a += h + m + l
+RF_DEV void rf_tf_add2(RfTf2& a, unsigned long long h, unsigned long long m, unsigned long long l)
 {
-    const unsigned hb = __float_as_uint(hi);
-    unsigned long long m = rf_df_int(hi, lo);
-    if (m == 0) return 0ULL;
-    int E = (int)(hb >> 23) - 127 + 1023;
-    if (!(m >> 52)) m <<= 1, E--;
-    return ((unsigned long long)E << 52) + (m - (1ULL << 52));
+    unsigned long long e1, e2, e3;
+    rf_two_sum2(a.h, h, a.h, e1);
+    rf_two_sum2(a.m, m, a.m, e2);
+    rf_two_sum2(a.m, e1, a.m, e3);
+    a.l = rf_add2(rf_add2(a.l, l), rf_add2(e2, e3));
+}
+
+// The double nearest hi + mid + lo, as bits, with integer and FP32 instructions only: hi 0 or a normal
+// float in [2^-103, 2^127), mid at most half a unit of hi's last place, lo of mid's.  In units of
+// 2^(eh - 179), where eh is hi's biased exponent, hi is a whole number of 53 bits; of half that where hi is
+// a power of two and mid is below 0, so that the sum has 53 bits too.  mid and lo are scaled by two
+// powers of two that are floats, exactly (products below 2^-126 aside, which no rounding depends on);
+// mid's nearest whole number leaves at most half a unit, which is rounded together with lo.
+RF_DEV unsigned long long rf_tf_to_f64(float hi, float mid, float lo)
+{
+    const unsigned hb = __float_as_uint(hi), eh = hb >> 23, half = (hb & 0x7FFFFFu) == 0u && mid < 0.f ? 1u : 0u;
+    const bool small = eh < 64u;
+    const float s1 = small ? 0x1p60f : 1.f, s2 = __uint_as_float((306u + half - eh - (small ? 60u : 0u)) << 23);
+    const float x = __fmul_rn(__fmul_rn(mid, s1), s2), y = __fmul_rn(__fmul_rn(lo, s1), s2);
+    const int i = __float2int_rn(x);
+    const int k = __float2int_rn(__fadd_rn(__fsub_rn(x, __int2float_rn(i)), y));
+    const unsigned long long m = ((unsigned long long)((hb & 0x7FFFFFu) | 0x800000u) << (29 + half)) + (unsigned long long)(long long)(i + k);
+    // m is in [2^52, 2^53]; 2^53 carries into the exponent
+    return hb ? ((unsigned long long)(eh + 896u - half) << 52) + (m - (1ULL << 52)) : 0ULL;
+}
+
+RF_DEV unsigned long long rf_df_to_f64(float hi, float lo) { return rf_tf_to_f64(hi, lo, 0.f); }
+
+// the doubles nearest the two sums, as bits (their parts are renormalised first)
+RF_DEV ulonglong2 rf_tf2_to_f64(const RfTf2& a)
+{
+    unsigned long long h, m, l;
+    rf_two_sum2(a.h, a.m, h, m);
+    rf_two_sum2(m, a.l, m, l);
+    rf_two_sum2(h, m, h, m);  // (where a.l is above a unit of a.m's)
+    float h0, h1, m0, m1, l0, l1;
+    rf_unf2(h, h0, h1);
+    rf_unf2(m, m0, m1);
+    rf_unf2(l, l0, l1);
+    return make_ulonglong2(rf_tf_to_f64(h0, m0, l0), rf_tf_to_f64(h1, m1, l1));
 }
 
 // ---------------------------------------------------------------------------------------
