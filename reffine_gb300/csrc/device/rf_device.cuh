@@ -314,33 +314,13 @@ RF_DEV double rf_u2f(unsigned long long x) { return __longlong_as_double((long l
 // floats hi + lo (a "double-float", 48 significant bits) while its addends are non-negative: each
 // addend is split into two floats with integer operations only, and added with the error-free
 // two-sum of Knuth (TAOCP vol. 2, 4.2.2) and Dekker's renormalisation (as in the double-float
-// additions of Hida, Li and Bailey's QD library): the pair stays within about 2^-46 of the exact
+// additions of Hida, Li and Bailey's QD library): the pair stays within a few 2^-47 of the exact
 // running sum, relative to the sum.
 // FP64 sums of the same rows in another order differ by the same order of rounding, far inside
 // the 1e-12 relative tolerance kept against the serial reference loop.
 // A slot's 64 bits hold the pair (hi in the low word, lo in the high word); +0.0 is all zeros in
 // both encodings.
 // ---------------------------------------------------------------------------------------
-
-// v = hi + lo for a non-negative v, 0 <= v - (hi + lo) < 2^-46 v; false (and nothing set) unless v
-// is +0 or a normal double in [2^-103, 2^91): negative values, -0, subnormals, larger values,
-// infinities and NaN are left to FP64 arithmetic.  hi takes the exponent and the leading 23
-// fraction bits of v (so hi is v truncated to 24 bits); lo the next 23 (the last 6 are dropped),
-// built as (1.m - 1.0) x 2^k from two floats with the same exponent, which subtract exactly.  One
-// unsigned compare on the high word tests sign and exponent together.  The dropped bits bias a
-// sum low by at most 2^-46 of it (2^-47 on average), 4500 times inside a 1e-12 tolerance.
-RF_DEV bool rf_df_split(double v, float& hi, float& lo)
-{
-    const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
-    // computed whatever the range (no branch), kept only in range
-    const bool in = h - (920u << 20) < (194u << 20);
-    const unsigned hb = __funnelshift_l(l, h - (896u << 20), 3);  // exponent - 896, 23 fraction bits
-    const unsigned c = (hb & 0x7F800000u) - (23u << 23);           // 2^(exponent of v - 23)
-    const float lf = __uint_as_float(c + ((l & 0x1FFFFFFFu) >> 6)) - __uint_as_float(c);
-    hi = in ? __uint_as_float(hb) : 0.f;
-    lo = in ? lf : 0.f;
-    return in || (h | l) == 0u;
-}
 
 RF_DEV void rf_two_sum(float a, float b, float& s, float& e)
 {
@@ -362,44 +342,35 @@ RF_DEV void rf_df_add_same_sign(float& ah, float& al, float bh, float bl)
     al = __fsub_rn(e, __fsub_rn(ah, s));
 }
 
-// one double-float slot update, in three steps the caller interleaves over a row's slots (so
-// their latencies overlap): split the addend, add it to the loaded pair, store.  rf_df_step
-// returns false, with nothing to store, when the addend is not a non-negative value in the
-// split's range: the caller then turns its slots into doubles and adds in FP64.  A slot so only
-// ever sums non-negative values, which keeps the sum well conditioned: its relative error stays
-// that of the additions (about 2^-48 times the square root of their number, typically), and it
-// cannot reach the float range (addends below 2^91; a thread adds fewer than 2^36 of them to a
-// slot in one work unit, far more rows than device memory holds).  Sums with negative addends,
-// where cancellation can occur, are left to FP64, whose error relative to the result is 32 times
-// smaller.
-RF_DEV bool rf_df_step(float2 a, double v, float2& out)
-{
-    float bh, bl;
-    const bool ok = rf_df_split(v, bh, bl);
-    rf_df_add_same_sign(a.x, a.y, bh, bl);
-    out = a;
-    return ok;
-}
-
-// Two slots of neighbouring aggregates at once, for addends in the split's range (Z: or +0; checked
-// before, rf_df_in and rf_df_ok).  The low float is rounded here, not truncated: |v - (hi + lo)| is at
-// most 2^-47 v and has no bias.  The slots are kept as one float4 {hi0, hi1, lo0, lo1}, so that one 16-byte access
-// moves both and their high and low parts are register pairs for Blackwell's two-wide FP32
-// instructions (add.f32x2, sub.f32x2): the same additions, correctly rounded, in half the instructions.
+// Addends that a slot takes: normal doubles in [2^-103, 2^91), by one unsigned compare on the high word,
+// which tests sign and exponent together (rf_df_in), and +0 (rf_df_ok).  A negative addend, -0, a
+// subnormal, a larger value, an infinity or a NaN turns the thread's slots into doubles (rf_df_to_f64)
+// and the rest of its unit is summed in FP64.  A slot so only ever sums non-negative values, which
+// keeps the sum well conditioned: its relative error stays that of the additions (about 2^-48 times the
+// square root of their number, typically), and it cannot reach the float range (a thread adds fewer
+// than 2^36 of them to a slot in one work unit, far more rows than device memory holds).  Sums with
+// negative addends, where cancellation can occur, are left to FP64, whose error relative to the result
+// is 32 times smaller.
 RF_DEV bool rf_df_in(double v) { return (unsigned)__double2hiint(v) - (920u << 20) < (194u << 20); }
 
 RF_DEV bool rf_df_ok(double v) { return rf_df_in(v) || __double_as_longlong(v) == 0; }
 
+// v = hi + lo within 2^-47 v for an addend in the range (Z: or +0).  hi takes the exponent and the
+// leading 23 fraction bits of v, lo the next 23, rounded so that they have no bias, built as
+// (1.m - 1.0) x 2^k from two floats that subtract exactly.
 template <bool Z>
 RF_DEV void rf_df_split_in(double v, float& hi, float& lo)
 {
     const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
-    const unsigned hb = __funnelshift_l(l, h - (896u << 20), 3);  // as in rf_df_split
-    const unsigned c = (hb & 0x7F800000u) - (23u << 23);
+    const unsigned hb = __funnelshift_l(l, h - (896u << 20), 3);  // exponent - 896, 23 fraction bits
+    const unsigned c = (hb & 0x7F800000u) - (23u << 23);           // 2^(exponent of v - 23)
     hi = __uint_as_float(Z && h == 0u ? 0u : hb);
     lo = __uint_as_float(c + (((l & 0x1FFFFFFFu) + 32u) >> 6)) - __uint_as_float(c);  // 0 for +0
 }
 
+// Two slots of neighbouring aggregates are kept as one float4 {hi0, hi1, lo0, lo1}, so that one 16-byte
+// access moves both and their high and low parts are register pairs for Blackwell's two-wide FP32
+// instructions (add.f32x2, sub.f32x2): the same additions, correctly rounded, in half the instructions.
 RF_DEV unsigned long long rf_f2(float x, float y)
 {
     unsigned long long r;

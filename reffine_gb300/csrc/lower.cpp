@@ -2012,8 +2012,8 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         // the probes occupancy - the 200M-row join measured 1.11 -> 1.23 ms with it)
         auto emit_slot_add = [&](std::ostream& so, bool use_df) {
             // an addend that is negative or out of the double-float range turns every such slot of
-            // the thread into a double and the thread continues in FP64 (rf_df_step in
-            // rf_device.cuh); rf_slots_done leaves doubles in all slots for the block's fold
+            // the thread into a double and the thread continues in FP64 (rf_slot_add_some); where a
+            // thread of the block did, rf_slots_done leaves doubles in all slots for the block's fold
             std::vector<int> dfm;
             for (int m = 0; m < M; m++) {
                 auto& lf = leaves[g0[m]];
@@ -2529,7 +2529,6 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         int HK = 128;
         while (HK > 8 && HW * HK * LL * 8 > 16 * 1024) HK /= 2;
         plan_.hg_hot = HK;
-        plan_.hg_warm = 0;
         std::string sl = std::to_string(d.slot);
         std::string c0 = "P.t[" + sl + "].col[0]";
         std::ostringstream o;

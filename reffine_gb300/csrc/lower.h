@@ -88,7 +88,6 @@ struct Plan {
     int merge_vecs = 0;                 // merge join: vectors walked together
     int union_inputs[2] = {-1, -1};     // union merge: the two merged vectors (Func inputs)
     int hg_hot = 0;                     // hash group-by: hottest keys folded per warp (index 2x)
-    int hg_warm = 0;                    // hash group-by: further hot keys in shared memory (index 2x)
     int groups = 0, aggs = 0;           // grouped plans
     bool compact = false;               // grouped plans: rows are queued before their index probe
     int pref_threads = 256;             // the block size the plan runs fastest at, untuned

@@ -185,8 +185,7 @@ struct rf_plan {
     long long* d_res = nullptr;       // null count
     // hash group-by
     void* hg_keys = nullptr;
-    void* hg_acc = nullptr;
-    size_t hg_keys_cap = 0, hg_acc_cap = 0;
+    size_t hg_keys_cap = 0;
     long long hg_retry_cap = 0;
     int hg_factor_override = 0;       // set while the autotuner times a hash-table sizing
     void* hg_img = nullptr;           // hot-key image of the last input table (device)

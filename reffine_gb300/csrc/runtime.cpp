@@ -1191,7 +1191,6 @@ extern "C" int rf_plan_free(rf_plan* p)
     if (p->buf) cudaFreeAsync(p->buf, p->ctx->stream);
     cudaFree(p->d_tiles);
     cudaFree(p->hg_keys);
-    cudaFree(p->hg_acc);
     cudaFree(p->seg_woff);
     cudaFree(p->seg_tmp);
     cudaFree(p->seg_part);
@@ -2308,7 +2307,6 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         P.aux_n0 = n;
     }
     if (union_merge) {
-        // paired-row counts of the first vector, scanned in place (nA + 1 entries)
         rf_table* ta = args[pl.union_inputs[0]].table;
         rf_table* tb = args[pl.union_inputs[1]].table;
         if (!pl.vectorize && (ta->cols[0].valid || tb->cols[0].valid)) {
