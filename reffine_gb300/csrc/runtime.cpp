@@ -2157,6 +2157,50 @@ int ndv_estimate(rf_table* t, int col, cudaStream_t s, long long* out)
 
 }  // namespace rfrt
 
+namespace rfrt {
+TableScratch table_scratch(const rf_plan* p, const rf_arg* args, long long elements)
+{
+    const rfg::Plan& pl = p->plan;
+    TableScratch z;
+    auto tiles_of = [](long long n) { return (n + RF_MAT_TILE - 1) / RF_MAT_TILE; };
+    long long ntiles = std::max<long long>(tiles_of(elements), 1);
+    if (pl.kind == rfg::PlanKind::UNION_MERGE)  // (counts the second side's rows)
+        ntiles = std::max(ntiles, tiles_of(args[pl.union_inputs[1]].table->cols[0].nvals));
+    bool counts = false;
+    for (const auto& k : pl.kernels) counts = counts || k.role == rfg::KernelSpec::COUNT;
+    if (counts) {
+        z.bit_bytes = (size_t)ntiles * (RF_MAT_TILE / 8);
+        z.tiles = z.bit_bytes + (size_t)ntiles * 8;
+    }
+    if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
+        const rf_table* t = args[pl.drive_input].table;
+        const long long runs = t->cols[0].nvals;
+        z.rows = t->cols[0].logical;
+        for (int c : pl.cols_read[pl.drive_input])
+            if (c != 0) z.rows = std::min(z.rows, t->cols[c].nvals);
+        z.seg_tiles = (runs + z.rows + pl.seg_items - 1) / pl.seg_items;
+        z.bounds = (size_t)(z.seg_tiles + 1) * 8;
+        z.part = (size_t)(runs + z.seg_tiles + 1) * pl.acc_bytes;
+    }
+    if (pl.kind == rfg::PlanKind::MERGE_JOIN) {
+        // [tiles + 1][vectors] bounds; a partner row for each row of the first vector in each other one
+        z.bounds = (size_t)(ntiles + 1) * pl.merge_vecs * 8;
+        z.part = (size_t)std::max<long long>(elements, 1) * (pl.merge_vecs - 1) * 8;
+    }
+    if (pl.kind == rfg::PlanKind::UNION_MERGE) {
+        // the bounds of both sides' tiles, a word of prefix counts per 64 rows of the second side and
+        // the rows its unpaired ones follow
+        const long long nb = args[pl.union_inputs[1]].table->cols[0].nvals;
+        z.n0 = tiles_of(args[pl.union_inputs[0]].table->cols[0].nvals);
+        z.n1 = tiles_of(nb);
+        z.bounds = (size_t)(z.n0 + z.n1 + 2) * 16;
+        z.prefix = (size_t)(z.n1 + 1) * (RF_MAT_TILE / 16);
+        z.part = (size_t)(nb + 1) * 8;
+    }
+    return z;
+}
+}  // namespace rfrt
+
 namespace {
 
 // Runs an Op plan: allocates the output table (capacity = the loop's row range, so no 1e8-row
@@ -2166,20 +2210,31 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
 {
     rf_ctx* ctx = p->ctx;
     const rfg::Plan& pl = p->plan;
-    // a hash group-by's table lives for the run only (see below); an overflow's rerun grows it
-    // first, and whichever table is current when the outermost run returns goes back to the pool
-    struct ReleaseHashTable {
+    // What grows with the inputs lives for the run only: a serving mix holds thousands of plans (one
+    // per query's constants), and each keeping its hash table, say, measured 52 GB for 722 plans.  An
+    // overflow's rerun of a hash group-by grows its table first, and whichever is current when the
+    // outermost run returns goes back to the pool.  (Stream-ordered; a buffer of up to kKept bytes
+    // stays, so that a small query takes nothing from the pool.)
+    struct Release {
         rf_plan* p;
         cudaStream_t s;
-        ~ReleaseHashTable()
+        void give(void** buf, size_t* cap, size_t kept)
         {
-            if (p->hg_keys) cudaFreeAsync(p->hg_keys, s);
-            p->hg_keys = nullptr;
-            p->hg_keys_cap = 0;
+            if (*cap <= kept) return;
+            if (*buf) cudaFreeAsync(*buf, s);
+            *buf = nullptr;
+            *cap = 0;
         }
-    };
-    std::unique_ptr<ReleaseHashTable> release_hash;
-    if (pl.kind == rfg::PlanKind::HASH_GROUP) release_hash.reset(new ReleaseHashTable{p, s});
+        ~Release()
+        {
+            constexpr size_t kKept = 64 << 10;
+            give(&p->hg_keys, &p->hg_keys_cap, 0);
+            give((void**)&p->d_tiles, &p->tiles_cap, kKept);
+            give((void**)&p->seg_woff, &p->seg_runs_cap, kKept);
+            give((void**)&p->seg_tmp, &p->seg_tmp_cap, kKept);
+            give(&p->seg_part, &p->seg_part_cap, kKept);
+        }
+    } release{p, s};
     RfParams P;
     long long lo, hi;
     int rc = fill_params(p, args, n_args, P, lo, hi, true);
@@ -2196,10 +2251,7 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         hg_cap = std::max<long long>(1024, (long long)((double)factor / 100.0 * (double)ndv));
         if (p->hg_retry_cap > hg_cap) hg_cap = p->hg_retry_cap;
         hg_cap = (hg_cap + 3) & ~3LL;  // whole sectors of keys
-        // slots of pl.acc_bytes bytes: keys, accumulators (and up to 64 bytes between).  The table is
-        // taken from the pool for this run and handed back when the run ends (stream-ordered):
-        // a serving mix holds thousands of hash group-by plans (one per query's constants), and
-        // each keeping its table measured 52 GB for 722 plans.
+        // slots of pl.acc_bytes bytes: keys, accumulators (and up to 64 bytes between)
         if (!grow(&p->hg_keys, &p->hg_keys_cap, (size_t)(hg_cap + 1) * pl.acc_bytes + 64, s))
             return fail(ctx, RF_ERR_OOM, "hash table allocation (%lld slots)", hg_cap);
         P.aux4 = p->hg_keys;
@@ -2257,11 +2309,13 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         return rc;
     }
     long long ntiles = (hi - lo + P.tile_rows - 1) / P.tile_rows;
-    // [a bit per element, whole tiles][count / offset of each tile]
-    const size_t bit_bytes = (size_t)std::max<long long>(ntiles, 1) * (RF_MAT_TILE / 8);
-    if (!grow((void**)&p->d_tiles, &p->tiles_cap, bit_bytes + (size_t)std::max<long long>(ntiles, 1) * 8, s)) {
+    const rfrt::TableScratch z = rfrt::table_scratch(p, args, hi - lo);
+    if ((z.tiles && !grow((void**)&p->d_tiles, &p->tiles_cap, z.tiles, s)) ||
+        (z.bounds && !grow((void**)&p->seg_woff, &p->seg_runs_cap, z.bounds, s)) ||
+        (z.prefix && !grow((void**)&p->seg_tmp, &p->seg_tmp_cap, z.prefix, s)) ||
+        (z.part && !grow(&p->seg_part, &p->seg_part_cap, z.part, s))) {
         free_table_mem(t.get());
-        return fail(ctx, RF_ERR_OOM, "tile buffer allocation failed");
+        return fail(ctx, RF_ERR_OOM, "scratch of a table result (%zu bytes)", z.bytes());
     }
     // rows written and nulls: a compaction's last block leaves its count in pinned host memory; the
     // null rows of a vectorised one are counted with atomics, on the device
@@ -2273,61 +2327,33 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     for (int i = 0; i < 4; i++) h_counts[i] = 0;
     if (pl.vectorize) CUDA_TRY(ctx, cudaMemsetAsync(p->d_res, 0, 64, s));
     P.aux1 = p->d_tiles;
-    P.aux2 = (unsigned char*)p->d_tiles + bit_bytes;
+    P.aux2 = (unsigned char*)p->d_tiles + z.bit_bytes;
     P.aux3 = p->d_res;
     P.host_rows = (long long*)p->h_res;
-    long long seg_tiles = 0;
+    const long long seg_tiles = z.seg_tiles;
     if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
-        rf_table* vt = args[pl.drive_input].table;
-        const long long nruns = vt->cols[0].nvals;
-        long long nrows = vt->cols[0].logical;
-        for (int c : pl.cols_read[pl.drive_input])
-            if (c != 0) nrows = std::min(nrows, vt->cols[c].nvals);
-        seg_tiles = (nruns + nrows + pl.seg_items - 1) / pl.seg_items;
-        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(seg_tiles + 1) * 8, s) ||
-            !grow(&p->seg_part, &p->seg_part_cap, (size_t)(nruns + seg_tiles + 1) * pl.acc_bytes, s)) {
-            free_table_mem(t.get());
-            return fail(ctx, RF_ERR_OOM, "segmented-reduce buffers");
-        }
         P.aux4 = p->seg_woff;
         P.aux5 = p->seg_part;
-        P.aux_n0 = nrows;
+        P.aux_n0 = z.rows;
         P.aux_n1 = seg_tiles;
     }
     if (pl.kind == rfg::PlanKind::MERGE_JOIN) {
-        // [tiles + 1][vectors] bounds; a partner row for each row of the first vector in each other one
-        const long long n = std::max<long long>(hi - lo, 1);
-        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(ntiles + 1) * pl.merge_vecs * 8, s) ||
-            !grow(&p->seg_part, &p->seg_part_cap, (size_t)n * (pl.merge_vecs - 1) * 8, s)) {
-            free_table_mem(t.get());
-            return fail(ctx, RF_ERR_OOM, "merge buffers");
-        }
         P.aux4 = p->seg_woff;
         P.aux5 = p->seg_part;
-        P.aux_n0 = n;
+        P.aux_n0 = std::max<long long>(hi - lo, 1);
     }
     if (union_merge) {
-        rf_table* ta = args[pl.union_inputs[0]].table;
-        rf_table* tb = args[pl.union_inputs[1]].table;
-        if (!pl.vectorize && (ta->cols[0].valid || tb->cols[0].valid)) {
+        if (!pl.vectorize &&
+            (args[pl.union_inputs[0]].table->cols[0].valid || args[pl.union_inputs[1]].table->cols[0].valid)) {
             free_table_mem(t.get());
             return fail(ctx, RF_ERR_UNSUPPORTED,
                         "a union over iterator columns with nulls is lowered in the vectorised form only");
         }
-        // tiles of each side, the bounds of both, a word of prefix counts per 64 rows of the second
-        // side and the rows its unpaired ones follow
-        const long long nb = tb->cols[0].nvals;
-        P.aux_n0 = (ta->cols[0].nvals + RF_MAT_TILE - 1) / RF_MAT_TILE;
-        P.aux_n1 = (nb + RF_MAT_TILE - 1) / RF_MAT_TILE;
-        if (!grow((void**)&p->seg_woff, &p->seg_runs_cap, (size_t)(P.aux_n0 + P.aux_n1 + 2) * 16, s) ||
-            !grow((void**)&p->seg_tmp, &p->seg_tmp_cap, (size_t)(P.aux_n1 + 1) * (RF_MAT_TILE / 16), s) ||
-            !grow(&p->seg_part, &p->seg_part_cap, (size_t)(nb + 1) * 8, s)) {
-            free_table_mem(t.get());
-            return fail(ctx, RF_ERR_OOM, "union merge buffers");
-        }
-        P.aux4 = p->seg_woff;
         P.aux0 = p->seg_tmp;
+        P.aux4 = p->seg_woff;
         P.aux5 = p->seg_part;
+        P.aux_n0 = z.n0;
+        P.aux_n1 = z.n1;
     }
     int units = units_for(p, ntiles);
     P.nunits = units;

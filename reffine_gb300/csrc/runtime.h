@@ -17,6 +17,20 @@ int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, void* ou
 // fills the parameter block of a plan run; lo/hi = tiling range
 int fill_params(rf_plan* p, const rf_arg* args, int n_args, RfParams& P, long long& lo, long long& hi,
                 bool may_allocate);
+// Device buffers of a table-result run over `elements` elements (a hash group-by's slots, else the
+// tiling range) that grow with its inputs.  They live for the run (see run_table); a server counts
+// them before it admits one.
+struct TableScratch {
+    size_t tiles = 0;      // a bit per element, then a count / offset a tile
+    size_t bit_bytes = 0;  // of which the bits
+    size_t bounds = 0;     // tile bounds of a run-end grouping or a merge
+    size_t prefix = 0;     // an outer merge's prefix counts
+    size_t part = 0;       // a run-end grouping's states, a merge's partner rows
+    long long rows = 0, seg_tiles = 0;  // a run-end grouping's rows and tiles
+    long long n0 = 0, n1 = 0;           // an outer merge's tiles of each side
+    size_t bytes() const { return tiles + bounds + prefix + part; }
+};
+TableScratch table_scratch(const rf_plan* p, const rf_arg* args, long long elements);
 // one host-to-device copy that upload() leaves to its caller (see `defer`)
 struct HostCopy {
     void* dst;

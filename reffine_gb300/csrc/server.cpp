@@ -69,7 +69,7 @@ struct Lane {
 };
 
 // device scratch a request holds while in flight
-size_t footprint_of(rf_plan* p, long long lo, long long hi)
+size_t footprint_of(rf_plan* p, const rf_arg* args, long long lo, long long hi)
 {
     const rfg::Plan& pl = p->plan;
     long long rows = std::max<long long>(hi - lo, 0);
@@ -81,8 +81,12 @@ size_t footprint_of(rf_plan* p, long long lo, long long hi)
     }
     size_t row_bytes = 8;
     for (auto& c : pl.out_cols) row_bytes += c.size();
-    size_t bytes = (size_t)rows * row_bytes + (size_t)(rows / pl.tile_rows + 2) * (8 + RF_MAT_TILE / 8);
-    if (pl.kind == rfg::PlanKind::HASH_GROUP) bytes += (size_t)rows * 2 * (8 + pl.acc_bytes);
+    size_t bytes = (size_t)rows * row_bytes;
+    if (pl.kind == rfg::PlanKind::HASH_GROUP) {  // (its elements are slots: two a row and more at most)
+        bytes += (size_t)rows * 2 * (8 + pl.acc_bytes);
+        rows = rows * 11 / 5 + 1024;
+    }
+    bytes += rfrt::table_scratch(p, args, rows).bytes();
     return bytes;
 }
 
@@ -366,7 +370,7 @@ extern "C" int rf_server_submit(rf_server* S, rf_plan* plan, const rf_arg* args,
     long long lo, hi;
     int rc = fill_params(plan, args, n_args, P, lo, hi, false);
     if (rc) return rc;
-    r.footprint = footprint_of(plan, lo, hi);
+    r.footprint = footprint_of(plan, args, lo, hi);
     // batched: Reduce plans with host-known loop bounds; the rest run on the solo lane
     bool batched = S->cfg.mode == RF_SERVE_BATCHED && plan->batch_fn;
     std::lock_guard<std::mutex> lk(S->mu);
