@@ -2474,6 +2474,14 @@ extern "C" int rf_plan_run_noalloc(rf_plan* p, const rf_arg* args, int32_t n_arg
     size_t out_bytes = (pl.out_size + 255) / 256 * 256;
     size_t acc = pl.acc_bytes ? pl.acc_bytes : 8;
     size_t need = out_at + out_bytes + (size_t)units * acc;
+    if (need > cap && P.tile_rows < pl.tile_rows) {
+        // an untuned tiling cuts a small table into more units than the plan's own tiles, whose
+        // partial sums may fit where those of more units do not
+        P.tile_rows = pl.tile_rows;
+        ntiles = (hi - lo + P.tile_rows - 1) / P.tile_rows;
+        units = units_for(p, ntiles);
+        need = out_at + out_bytes + (size_t)units * acc;
+    }
     if (need > cap)
         return fail(ctx, RF_ERR_INVALID,
                     "rf_plan_run_noalloc: this run needs %zu bytes of scratch, the fixed array holds %zu "
