@@ -2361,8 +2361,11 @@ extern "C" __global__ void __launch_bounds__(256) rf_ixf_build(const __grid_cons
         plan_.acc_bytes = (size_t)G * M * 8;
         plan_.compact = compact;
         // Double-float sums run faster in blocks of 512 threads, where their slots fit one: the rows of a
-        // step are held in 104 registers a thread instead of 80 (the 6-group group-by, each at its best
-        // tile: 60M rows 548 us against 591 us at 256 threads, 6M 84 / 107, 1M 37 / 47, 100K 29 / 29)
+        // step are held in 104 registers a thread instead of 80, though plans of few slots keep 16 warps
+        // an SM so instead of 24 (untuned, 256 / 512 threads: the 6-group group-by of 36 slots, 60M rows
+        // 570 / 523 us, 6M 92 / 73, 1M 43 / 27, 100K 23 / 21; 10M rows of 4 groups of double sums in 4
+        // slots 36.8 / 34.9, 8 45.5 / 45.3, 12 59.6 / 57.5, 24 95.9 / 100.6, 48 174.6 / 164.0, and 1M rows
+        // 10.3 / 10.3, 13.9 / 12.4, 17.7 / 16.4, 24.7 / 18.2, 43.1 / 30.9)
         const size_t smem512 = (size_t)G * M * 512 * 8;
         if (!compact && o.str().find("rf_slots_to_f64") != std::string::npos && smem512 <= 200 * 1024) plan_.pref_threads = 512;
     }

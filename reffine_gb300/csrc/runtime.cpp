@@ -1250,18 +1250,18 @@ int hg_factor_for(rf_plan* p, long long rows)
 }
 
 // The tiling of a scan that was not tuned: tiles that give the resident blocks the same number of
-// rows, so that no last wave is partly filled and a small table uses the whole GPU (8192-row tiles
-// left 2 blocks for 10K rows, 123 for 1M, and 17 tiles to some units and 16 to others at 60M).
+// rows, so that no last wave is partly filled (8192-row tiles left 123 blocks for 1M rows, and 17 tiles to
+// some units and 16 to others at 60M), but not units so small that their folds cost more than they share.
 long long untuned_tile_rows(rf_plan* p, long long rows)
 {
     const rfg::Plan& pl = p->plan;
-    const long long T = pl.threads, wave = std::max(1, p->max_units), sms = std::max(1, p->ctx->sm_count);
+    const long long T = pl.threads, wave = std::max(1, p->max_units);
     auto up = [](long long x, long long m) { return (std::max(x, 1LL) + m - 1) / m * m; };
     auto share = [&](long long units) { return (std::max(rows, 1LL) + units - 1) / units; };
     if (pl.kind == rfg::PlanKind::SCAN_REDUCE) {
-        // one unit to a resident block; a table of less than 4096 rows to each takes about two units an
-        // SM, of two 4-row steps of their threads at least (filter+sum, 8192-row tiles / these: 10K rows
-        // 13.3 / 8.2 us, 100K 14.4 / 8.3, 1M 15.2 / 12.3, 6M 45.3 / 34.2, 50M 216 / 207)
+        // one unit to a resident block, of 4096 rows at least: four 4-row steps of its threads
+        // (filter+sum, launched, 8192-row tiles / these: 10K rows 13.6 / 10.3 us, 100K 14.5 / 10.3,
+        // 1M 14.5 / 12.3, 6M 45.5 / 33.5, 50M 217 / 206)
         return std::max(up(share(wave), 4), 4096LL);
     }
     if (pl.compact) {
