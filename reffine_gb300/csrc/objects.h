@@ -180,12 +180,10 @@ struct rf_plan {
     size_t batch_smem = 0;
     int batch_threads = 0;
     // table outputs
-    long long* d_tiles = nullptr;     // a bit per element, then per-tile counts / offsets
-    size_t tiles_cap = 0;             // bytes
+    void* scratch = nullptr;          // a run's scratch (kept between runs where it is small)
+    size_t scratch_cap = 0;           // bytes
     long long* d_res = nullptr;       // null count
     // hash group-by
-    void* hg_keys = nullptr;
-    size_t hg_keys_cap = 0;
     long long hg_retry_cap = 0;
     int hg_factor_override = 0;       // set while the autotuner times a hash-table sizing
     void* hg_img = nullptr;           // hot-key image of the last input table (device)
@@ -201,11 +199,6 @@ struct rf_plan {
     unsigned long long ixf_buf_for = 0;
     RfIndex ixf_ix{};
     cudaEvent_t ixf_ev = nullptr;     // recorded after the last run that read ixf_buf
-    // segmented reduce: tile bounds, states; merges: tile bounds, partner rows
-    long long* seg_woff = nullptr;
-    long long* seg_tmp = nullptr;
-    void* seg_part = nullptr;
-    size_t seg_runs_cap = 0, seg_part_cap = 0, seg_tmp_cap = 0;
 };
 
 // Work units of a value reduce over `ntiles` tiles: up to kUnitWaves waves of resident blocks.

@@ -1189,11 +1189,7 @@ extern "C" int rf_plan_free(rf_plan* p)
     }
     cudaStreamSynchronize(p->ctx->stream);
     if (p->buf) cudaFreeAsync(p->buf, p->ctx->stream);
-    cudaFree(p->d_tiles);
-    cudaFree(p->hg_keys);
-    cudaFree(p->seg_woff);
-    cudaFree(p->seg_tmp);
-    cudaFree(p->seg_part);
+    cudaFree(p->scratch);
     cudaFree(p->hg_img);
     cudaFreeHost(p->h_res);
     for (auto* t : p->staging)
@@ -2197,6 +2193,7 @@ TableScratch table_scratch(const rf_plan* p, const rf_arg* args, long long eleme
         z.prefix = (size_t)(z.n1 + 1) * (RF_MAT_TILE / 16);
         z.part = (size_t)(nb + 1) * 8;
     }
+    for (size_t* b : {&z.tiles, &z.bounds, &z.prefix, &z.part}) *b = (*b + 255) / 256 * 256;
     return z;
 }
 }  // namespace rfrt
@@ -2210,29 +2207,21 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
 {
     rf_ctx* ctx = p->ctx;
     const rfg::Plan& pl = p->plan;
-    // What grows with the inputs lives for the run only: a serving mix holds thousands of plans (one
-    // per query's constants), and each keeping its hash table, say, measured 52 GB for 722 plans.  An
-    // overflow's rerun of a hash group-by grows its table first, and whichever is current when the
-    // outermost run returns goes back to the pool.  (Stream-ordered; a buffer of up to kKept bytes
-    // stays, so that a small query takes nothing from the pool.)
+    // The scratch lives for the run only: a serving mix holds thousands of plans (one per query's
+    // constants), and each keeping its hash table, say, measured 52 GB for 722 plans.  An overflow's
+    // rerun of a hash group-by grows it first, and whichever is current when the outermost run returns
+    // goes back to the pool, in stream order.  (Up to kKept bytes stay, so that a small query takes
+    // nothing from the pool.)
     struct Release {
         rf_plan* p;
         cudaStream_t s;
-        void give(void** buf, size_t* cap, size_t kept)
-        {
-            if (*cap <= kept) return;
-            if (*buf) cudaFreeAsync(*buf, s);
-            *buf = nullptr;
-            *cap = 0;
-        }
         ~Release()
         {
-            constexpr size_t kKept = 64 << 10;
-            give(&p->hg_keys, &p->hg_keys_cap, 0);
-            give((void**)&p->d_tiles, &p->tiles_cap, kKept);
-            give((void**)&p->seg_woff, &p->seg_runs_cap, kKept);
-            give((void**)&p->seg_tmp, &p->seg_tmp_cap, kKept);
-            give(&p->seg_part, &p->seg_part_cap, kKept);
+            constexpr size_t kKept = 1 << 20;
+            if (p->scratch_cap <= kKept) return;
+            if (p->scratch) cudaFreeAsync(p->scratch, s);
+            p->scratch = nullptr;
+            p->scratch_cap = 0;
         }
     } release{p, s};
     RfParams P;
@@ -2240,6 +2229,7 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     int rc = fill_params(p, args, n_args, P, lo, hi, true);
     if (rc) return rc;
     long long hg_cap = 0;
+    size_t hash_bytes = 0;
     if (pl.kind == rfg::PlanKind::HASH_GROUP) {
         // hash table of hg_factor_for() slots per 100 estimated distinct keys (default 220: load
         // 0.45, i.e. 0.5 with a 10% margin on the estimate); a probe overflow reruns with twice
@@ -2252,9 +2242,7 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         if (p->hg_retry_cap > hg_cap) hg_cap = p->hg_retry_cap;
         hg_cap = (hg_cap + 3) & ~3LL;  // whole sectors of keys
         // slots of pl.acc_bytes bytes: keys, accumulators (and up to 64 bytes between)
-        if (!grow(&p->hg_keys, &p->hg_keys_cap, (size_t)(hg_cap + 1) * pl.acc_bytes + 64, s))
-            return fail(ctx, RF_ERR_OOM, "hash table allocation (%lld slots)", hg_cap);
-        P.aux4 = p->hg_keys;
+        hash_bytes = ((size_t)(hg_cap + 1) * pl.acc_bytes + 64 + 255) / 256 * 256;
         P.aux_n0 = vt->cols[0].logical;
         P.aux_n1 = hg_cap;
         if ((rc = hot_image(p, vt, s, &P.aux5))) return rc;
@@ -2309,14 +2297,23 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
         return rc;
     }
     long long ntiles = (hi - lo + P.tile_rows - 1) / P.tile_rows;
+    // one buffer: [hash table][bits, counts][tile bounds][prefix counts][states or partner rows]
     const rfrt::TableScratch z = rfrt::table_scratch(p, args, hi - lo);
-    if ((z.tiles && !grow((void**)&p->d_tiles, &p->tiles_cap, z.tiles, s)) ||
-        (z.bounds && !grow((void**)&p->seg_woff, &p->seg_runs_cap, z.bounds, s)) ||
-        (z.prefix && !grow((void**)&p->seg_tmp, &p->seg_tmp_cap, z.prefix, s)) ||
-        (z.part && !grow(&p->seg_part, &p->seg_part_cap, z.part, s))) {
+    if (hash_bytes + z.bytes() && !grow(&p->scratch, &p->scratch_cap, hash_bytes + z.bytes(), s)) {
         free_table_mem(t.get());
-        return fail(ctx, RF_ERR_OOM, "scratch of a table result (%zu bytes)", z.bytes());
+        return fail(ctx, RF_ERR_OOM, "scratch of a table result (%zu bytes)", hash_bytes + z.bytes());
     }
+    unsigned char* at = (unsigned char*)p->scratch;
+    if (pl.kind == rfg::PlanKind::HASH_GROUP) P.aux4 = at;
+    at += hash_bytes;
+    P.aux1 = at;
+    P.aux2 = at + z.bit_bytes;
+    at += z.tiles;
+    if (z.bounds) P.aux4 = at;
+    at += z.bounds;
+    if (z.prefix) P.aux0 = at;
+    at += z.prefix;
+    if (z.part) P.aux5 = at;
     // rows written and nulls: a compaction's last block leaves its count in pinned host memory; the
     // null rows of a vectorised one are counted with atomics, on the device
     if ((rc = result_buffer(p))) {
@@ -2326,22 +2323,14 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
     volatile long long* h_counts = (volatile long long*)p->h_res;
     for (int i = 0; i < 4; i++) h_counts[i] = 0;
     if (pl.vectorize) CUDA_TRY(ctx, cudaMemsetAsync(p->d_res, 0, 64, s));
-    P.aux1 = p->d_tiles;
-    P.aux2 = (unsigned char*)p->d_tiles + z.bit_bytes;
     P.aux3 = p->d_res;
     P.host_rows = (long long*)p->h_res;
     const long long seg_tiles = z.seg_tiles;
     if (pl.kind == rfg::PlanKind::SEG_REDUCE) {
-        P.aux4 = p->seg_woff;
-        P.aux5 = p->seg_part;
         P.aux_n0 = z.rows;
         P.aux_n1 = seg_tiles;
     }
-    if (pl.kind == rfg::PlanKind::MERGE_JOIN) {
-        P.aux4 = p->seg_woff;
-        P.aux5 = p->seg_part;
-        P.aux_n0 = std::max<long long>(hi - lo, 1);
-    }
+    if (pl.kind == rfg::PlanKind::MERGE_JOIN) P.aux_n0 = std::max<long long>(hi - lo, 1);
     if (union_merge) {
         if (!pl.vectorize &&
             (args[pl.union_inputs[0]].table->cols[0].valid || args[pl.union_inputs[1]].table->cols[0].valid)) {
@@ -2349,9 +2338,6 @@ int run_table(rf_plan* p, const rf_arg* args, int n_args, rf_table** out, cudaSt
             return fail(ctx, RF_ERR_UNSUPPORTED,
                         "a union over iterator columns with nulls is lowered in the vectorised form only");
         }
-        P.aux0 = p->seg_tmp;
-        P.aux4 = p->seg_woff;
-        P.aux5 = p->seg_part;
         P.aux_n0 = z.n0;
         P.aux_n1 = z.n1;
     }

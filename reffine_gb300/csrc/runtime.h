@@ -18,8 +18,8 @@ int enqueue(rf_plan* p, const rf_arg* args, int n_args, cudaStream_t s, void* ou
 int fill_params(rf_plan* p, const rf_arg* args, int n_args, RfParams& P, long long& lo, long long& hi,
                 bool may_allocate);
 // Device buffers of a table-result run over `elements` elements (a hash group-by's slots, else the
-// tiling range) that grow with its inputs.  They live for the run (see run_table); a server counts
-// them before it admits one.
+// tiling range) that grow with its inputs, in multiples of 256 bytes.  They live for the run (see
+// run_table); a server counts them before it admits one.
 struct TableScratch {
     size_t tiles = 0;      // a bit per element, then a count / offset a tile
     size_t bit_bytes = 0;  // of which the bits
